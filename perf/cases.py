@@ -343,7 +343,7 @@ def work(case):
         return {"bytes": 16 * valid * n + 16 * ghost, "flops": 28 * valid * n}
     if kind == "multigrid":
         helm = case["form"] == "helmholtz"
-        cycles = 5 if helm else 15
+        cycles = 15
         cells = case["n"] ** 3 * 8 / 7
         item = 4 if case["precision"] == "mixed" else 8
         return {"bytes": cycles * cells * item * (4 if helm else 3), "flops": cycles * cells * 9 * (22 if helm else 16)}
