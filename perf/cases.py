@@ -314,8 +314,7 @@ def run(s):
         s["engine"].submit(n, rhs, out, form=pb.MG_HELMHOLTZ if helm else pb.MG_POISSON, alpha=alpha)
     s["engine"].run_until_idle()
     s["engine"].poll()
-    # one array: the solutions of all requests, one after another
-    return np.concatenate([q[4] for q in s["requests"]])
+    return [q[4] for q in s["requests"]]
 
 
 def work(case):
@@ -572,4 +571,4 @@ def exact(case, seed):
         levels = (n & -n).bit_length() - 1
         a = torch.full_like(f, alpha) if helm else None
         out.append(_VCycle(n, levels, a, False).solve(f, 1e-8, 100).reshape(-1).cpu().numpy())
-    return np.concatenate(out)
+    return out
