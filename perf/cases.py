@@ -374,7 +374,7 @@ def tolerance(case):
     if kind == "multigrid":
         return {"rel": 1.5e-13} if fp64 else {"rel": 1e-12 if case["form"] == "helmholtz" else 4e-7}
     if kind == "serve":
-        return {"rel": 1.5e-13} if fp64 else {"rel": 4e-7}
+        return {"rel": 1.5e-13} if fp64 else {"rel": 1e-6}
     return {"rel": {"transfer": 5e-16, "algebra": 1e-15, "boxop": 1e-15, "partial": 2e-15, "steps": 4e-15,
                     "fas": 3e-15}[kind]}
 
