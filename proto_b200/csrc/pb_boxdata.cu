@@ -7,96 +7,99 @@
 //   Reduction<T,OP,DEVICE> ............ include/base/Proto_Reduction.H:113-185,
 //                                       include/base/implem/Proto_ReductionImplem.H:108-192
 //   InterpStencil::Constant ........... include/base/implem/Proto_InterpStencilDefs.H:1-15
-// The reference launches one kernel per call with blocks of one x-row each; these kernels are
-// grid-stride loops over the flattened box with coalesced x-fastest accesses.
+// The reference launches one kernel per call with blocks of one x-row each; these kernels walk rows
+// with several planes' loads in flight.
 #include <cfloat>
 #include <cstring>
 
 #include "pb_internal.cuh"
 #include "pb_stencil_impl.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
-struct Region {
-    int lo[3];
-    int n[3];
-};
+template <int OP>
+__device__ __forceinline__ double apply_op(double d, double s)
+{
+    if (OP == PB_OP_ADD) return dadd(d, s);
+    if (OP == PB_OP_SUB) return dsub(d, s);
+    if (OP == PB_OP_MUL) return dmul(d, s);
+    if (OP == PB_OP_DIV) return ddiv(d, s);
+    return s;
+}
 
 // ---- dst op= src on a region (both fields addressed through their own boxes) -----------------
 template <int OP>
-__global__ void __launch_bounds__(256) k_binop(double* dst, Box3 db, const double* __restrict__ src, Box3 sb, Region r,
-                                               int shx, int shy, int shz, int ncomp)
+__global__ void __launch_bounds__(kWalkThreads) k_binop(FieldView<double> d, long long dvol, FieldView<const double> s,
+                                                        long long svol, Walk w, int ncomp)
 {
-    const long long total = (long long)r.n[0] * r.n[1] * r.n[2];
-    const long long dSx = bsize(db, 0), dSxy = bsize(db, 0) * bsize(db, 1), dvol = bvol(db);
-    const long long sSx = bsize(sb, 0), sSxy = bsize(sb, 0) * bsize(sb, 1), svol = bvol(sb);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = r.lo[0] + (int)(i % r.n[0]);
-        long long q = i / r.n[0];
-        int y = r.lo[1] + (int)(q % r.n[1]);
-        int z = r.lo[2] + (int)(q / r.n[1]);
-        // (x,y,z) is a source point; its destination is shifted
-        long long si = (x - sb.lo[0]) + sSx * (y - sb.lo[1]) + sSxy * (z - sb.lo[2]);
-        long long di = (x + shx - db.lo[0]) + dSx * (y + shy - db.lo[1]) + dSxy * (z + shz - db.lo[2]);
-        for (int c = 0; c < ncomp; c++) {
-            double s = src[si + c * svol];
-            double& d = dst[di + c * dvol];
-            if (OP == PB_OP_ADD) d = dadd(d, s);
-            else if (OP == PB_OP_SUB) d = dsub(d, s);
-            else if (OP == PB_OP_MUL) d = dmul(d, s);
-            else if (OP == PB_OP_DIV) d = ddiv(d, s);
-            else d = s;
-        }
+    for (int c = blockIdx.z; c < ncomp; c += gridDim.z) {
+        double* dp = d.p + c * dvol;
+        const double* sp = s.p + c * svol;
+        walk_rows(w, [&](int x, int y, int z, int planes) {
+            double* dq = dp + x + d.sy * y + d.sz * z;
+            const double* sq = sp + x + s.sy * y + s.sz * z;
+            double sv[kWalkZ], dv[kWalkZ];
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++)
+                if (k < planes) {
+                    sv[k] = sq[k * s.sz];
+                    if (OP != PB_OP_ASSIGN) dv[k] = dq[k * d.sz];
+                }
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++)
+                if (k < planes) dq[k * d.sz] = apply_op<OP>(OP != PB_OP_ASSIGN ? dv[k] : 0.0, sv[k]);
+        });
     }
 }
 
 template <int OP>
-__global__ void __launch_bounds__(256) k_scalar(double* dst, Box3 db, Region r, double v, int ncomp)
+__global__ void __launch_bounds__(kWalkThreads) k_scalar(FieldView<double> d, long long dvol, Walk w, double v, int ncomp)
 {
-    const long long total = (long long)r.n[0] * r.n[1] * r.n[2];
-    const long long dSx = bsize(db, 0), dSxy = bsize(db, 0) * bsize(db, 1), dvol = bvol(db);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = r.lo[0] + (int)(i % r.n[0]);
-        long long q = i / r.n[0];
-        int y = r.lo[1] + (int)(q % r.n[1]);
-        int z = r.lo[2] + (int)(q / r.n[1]);
-        long long di = (x - db.lo[0]) + dSx * (y - db.lo[1]) + dSxy * (z - db.lo[2]);
-        for (int c = 0; c < ncomp; c++) {
-            double& d = dst[di + c * dvol];
-            if (OP == PB_OP_ADD) d = dadd(d, v);
-            else if (OP == PB_OP_SUB) d = dsub(d, v);
-            else if (OP == PB_OP_MUL) d = dmul(d, v);
-            else if (OP == PB_OP_DIV) d = ddiv(d, v);
-            else d = v;
-        }
+    for (int c = blockIdx.z; c < ncomp; c += gridDim.z) {
+        double* dp = d.p + c * dvol;
+        walk_rows(w, [&](int x, int y, int z, int planes) {
+            double* dq = dp + x + d.sy * y + d.sz * z;
+            double dv[kWalkZ];
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++)
+                if (OP != PB_OP_ASSIGN && k < planes) dv[k] = dq[k * d.sz];
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++)
+                if (k < planes) dq[k * d.sz] = apply_op<OP>(OP != PB_OP_ASSIGN ? dv[k] : 0.0, v);
+        });
     }
 }
 
 // forall body "out = a*x + b*y" (config: out = a*L(u) + b*u when Lu is materialised)
-__global__ void __launch_bounds__(256) k_axpby(double* out, Box3 ob, const double* __restrict__ xs, Box3 xb,
-                                               const double* __restrict__ ys, Box3 yb, Region r, double a, double b)
+__global__ void __launch_bounds__(kWalkThreads) k_axpby(FieldView<double> o, FieldView<const double> xs,
+                                                        FieldView<const double> ys, Walk w, double a, double b)
 {
-    const long long total = (long long)r.n[0] * r.n[1] * r.n[2];
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = r.lo[0] + (int)(i % r.n[0]);
-        long long q = i / r.n[0];
-        int y = r.lo[1] + (int)(q % r.n[1]);
-        int z = r.lo[2] + (int)(q / r.n[1]);
-        long long oi = (x - ob.lo[0]) + bsize(ob, 0) * ((y - ob.lo[1]) + bsize(ob, 1) * (long long)(z - ob.lo[2]));
-        long long xi = (x - xb.lo[0]) + bsize(xb, 0) * ((y - xb.lo[1]) + bsize(xb, 1) * (long long)(z - xb.lo[2]));
-        long long yi = (x - yb.lo[0]) + bsize(yb, 0) * ((y - yb.lo[1]) + bsize(yb, 1) * (long long)(z - yb.lo[2]));
-        out[oi] = dadd(dmul(a, xs[xi]), dmul(b, ys[yi]));
-    }
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        double* oq = o.p + x + o.sy * y + o.sz * z;
+        const double* xq = xs.p + x + xs.sy * y + xs.sz * z;
+        const double* yq = ys.p + x + ys.sy * y + ys.sz * z;
+        double xv[kWalkZ], yv[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) {
+                xv[k] = xq[k * xs.sz];
+                yv[k] = yq[k * ys.sz];
+            }
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) oq[k * o.sz] = dadd(dmul(a, xv[k]), dmul(b, yv[k]));
+    });
 }
 
 // ---- reductions ---------------------------------------------------------------------------------
-// Pass 1: every block folds its grid-stride share; pass 2 (the last block to finish, found through
-// an atomic ticket) folds the per-block partials in block order, so sums are deterministic.
+// Pass 1: every block folds its share; pass 2 (the last block to finish, found through an atomic
+// ticket) folds the per-block partials in block order, so sums are deterministic. A share is a fixed
+// set of tiles of kRedRows rows x kRedZ planes, walked like the pointwise kernels: each thread keeps
+// kRedZ loads in flight, one accumulator per plane of the tile.
 constexpr int kRedBlocks = 1024;
 constexpr int kRedThreads = 256;
+constexpr int kRedZ = 8;
 
 __device__ __forceinline__ double red_init(int op)
 {
@@ -138,20 +141,36 @@ __device__ double block_reduce(int op, double v)
     return v;
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_reduce(int op, const double* __restrict__ data, Box3 b, Region r,
-                                                        double* partials, unsigned int* ticket, double* result)
+// OP is a template argument so that the fold is one instruction or two, not a switch per cell.
+template <int op>
+__global__ void __launch_bounds__(kRedThreads) k_reduce(FieldView<const double> f, Walk w, double* partials,
+                                                        unsigned int* ticket, double* result)
 {
-    const long long total = (long long)r.n[0] * r.n[1] * r.n[2];
-    const long long Sx = bsize(b, 0), Sxy = bsize(b, 0) * bsize(b, 1);
-    double v = red_init(op);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = r.lo[0] + (int)(i % r.n[0]);
-        long long q = i / r.n[0];
-        int y = r.lo[1] + (int)(q % r.n[1]);
-        int z = r.lo[2] + (int)(q / r.n[1]);
-        v = red_upd(op, v, data[(x - b.lo[0]) + Sx * (y - b.lo[1]) + Sxy * (z - b.lo[2])]);
+    double acc[kRedZ];
+#pragma unroll
+    for (int k = 0; k < kRedZ; k++) acc[k] = red_init(op);
+    const int rows = kRedThreads >> w.lx;
+    const int lane = threadIdx.x & ((1 << w.lx) - 1), row = threadIdx.x >> w.lx;
+    const int ty = (w.ny + rows - 1) / rows, tz = (w.nz + kRedZ - 1) / kRedZ;
+    const long long tiles = (long long)ty * tz;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int y = (int)(t % ty) * rows + row, z = (int)(t / ty) * kRedZ;
+        if (y >= w.ny) continue;
+        const double* q = f.p + f.sy * y + f.sz * z;
+        const int planes = min(kRedZ, w.nz - z);
+        for (int x = lane; x < w.nx; x += 1 << w.lx) {
+            double v[kRedZ];
+#pragma unroll
+            for (int k = 0; k < kRedZ; k++)
+                if (k < planes) v[k] = __ldg(q + x + k * f.sz);
+#pragma unroll
+            for (int k = 0; k < kRedZ; k++)
+                if (k < planes) acc[k] = red_upd(op, acc[k], v[k]);
+        }
     }
+    double v = acc[0];
+#pragma unroll
+    for (int k = 1; k < kRedZ; k++) v = red_comb(op, v, acc[k]);
     v = block_reduce(op, v);
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -163,37 +182,48 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce(int op, const double* __
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double w = red_init(op);
+    double folded = red_init(op);
     // fixed order over the partials: thread k folds partials k, k+256, ... then the block tree
     for (int k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
         double p = ((volatile double*)partials)[k];
-        w = (k == threadIdx.x) ? p : red_comb(op, w, p);
+        folded = (k == threadIdx.x) ? p : red_comb(op, folded, p);
     }
-    if (threadIdx.x >= gridDim.x) w = red_init(op);
-    w = block_reduce(op, w);
+    if (threadIdx.x >= gridDim.x) folded = red_init(op);
+    folded = block_reduce(op, folded);
     if (threadIdx.x == 0) {
-        *result = w;
+        *result = folded;
         *ticket = 0;
     }
 }
 
 // ---- piecewise-constant prolongation ----------------------------------------------------------
-__global__ void __launch_bounds__(256) k_interp_const(int ratio, const double* __restrict__ src, Box3 sb, double* dst,
-                                                      Box3 db, Region r, int overwrite, double scale)
+// Fine cell p takes coarse cell floor(p / ratio). LR is log2(ratio) where that is a power of two (an
+// arithmetic shift floors like floor_div); -1 divides. Walked like the pointwise kernels; the four
+// planes' coarse and fine loads go out together. Measured (B200): AvgDown from 192^3, a copy of a 192^3
+// field and the prolongation added to it, 107 -> 67 us together with pb_stencil.cu's table kernel.
+template <int LR>
+__device__ __forceinline__ int coarse_of(int p, int ratio) { return LR >= 0 ? p >> (LR < 0 ? 0 : LR) : floor_div(p, ratio); }
+
+template <int LR>
+__global__ void __launch_bounds__(kWalkThreads) k_interp_const(int ratio, const double* __restrict__ src, Box3 sb,
+                                                               FieldView<double> d, Region r, Walk w, int overwrite,
+                                                               double scale)
 {
-    const long long total = (long long)r.n[0] * r.n[1] * r.n[2];
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = r.lo[0] + (int)(i % r.n[0]);
-        long long q = i / r.n[0];
-        int y = r.lo[1] + (int)(q % r.n[1]);
-        int z = r.lo[2] + (int)(q / r.n[1]);
-        int cx = floor_div(x, ratio), cy = floor_div(y, ratio), cz = floor_div(z, ratio);
-        double v = src[(cx - sb.lo[0]) + bsize(sb, 0) * ((cy - sb.lo[1]) + bsize(sb, 1) * (long long)(cz - sb.lo[2]))];
-        long long di = (x - db.lo[0]) + bsize(db, 0) * ((y - db.lo[1]) + bsize(db, 1) * (long long)(z - db.lo[2]));
-        double acc = overwrite ? 0.0 : dst[di];
-        dst[di] = dadd(acc, dmul(scale, v));
-    }
+    const long long Sx = bsize(sb, 0), Sxy = Sx * bsize(sb, 1);
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        const double* sq = src + (coarse_of<LR>(r.lo[0] + x, ratio) - sb.lo[0]) + Sx * (coarse_of<LR>(r.lo[1] + y, ratio) - sb.lo[1]);
+        double* dq = d.p + x + d.sy * y + d.sz * z;
+        double v[kWalkZ], acc[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) {
+                v[k] = __ldg(sq + Sxy * (coarse_of<LR>(r.lo[2] + z + k, ratio) - sb.lo[2]));
+                acc[k] = overwrite ? 0.0 : dq[k * d.sz];
+            }
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) dq[k * d.sz] = dadd(acc[k], dmul(scale, v[k]));
+    });
 }
 
 // ---- reduction scratch (per process, per device 0..15) ----------------------------------------
@@ -220,13 +250,6 @@ static int red_scratch(RedScratch** out)
     return PB_OK;
 }
 
-static inline Region region_of(const Box3& b)
-{
-    Region r;
-    for (int d = 0; d < 3; d++) { r.lo[d] = b.lo[d]; r.n[d] = (int)bsize(b, d); }
-    return r;
-}
-
 } // namespace pb
 
 using namespace pb;
@@ -239,15 +262,18 @@ int pb_boxdata_op_f64(int op, double* dst, pb_box dst_box, const double* src, pb
     Box3 db = to_box(dst_box), sb = to_box(src_box);
     Box3 r = intersect(db, sb);
     if (bempty(r)) return PB_OK;
-    Region rg = region_of(r);
+    const Region rg = region_of(r);
+    const Walk w = walk_of(rg);
+    const dim3 grid = walk_grid(w, ncomp);
+    const FieldView<double> d = view_of(dst, db, rg);
+    const FieldView<const double> sv = view_of(src, sb, rg);
     cudaStream_t st = (cudaStream_t)stream;
-    int grid = grid_for(bvol(r), 256);
     switch (op) {
-        case PB_OP_ADD: k_binop<PB_OP_ADD><<<grid, 256, 0, st>>>(dst, db, src, sb, rg, 0, 0, 0, ncomp); break;
-        case PB_OP_SUB: k_binop<PB_OP_SUB><<<grid, 256, 0, st>>>(dst, db, src, sb, rg, 0, 0, 0, ncomp); break;
-        case PB_OP_MUL: k_binop<PB_OP_MUL><<<grid, 256, 0, st>>>(dst, db, src, sb, rg, 0, 0, 0, ncomp); break;
-        case PB_OP_DIV: k_binop<PB_OP_DIV><<<grid, 256, 0, st>>>(dst, db, src, sb, rg, 0, 0, 0, ncomp); break;
-        default: k_binop<PB_OP_ASSIGN><<<grid, 256, 0, st>>>(dst, db, src, sb, rg, 0, 0, 0, ncomp); break;
+        case PB_OP_ADD: k_binop<PB_OP_ADD><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
+        case PB_OP_SUB: k_binop<PB_OP_SUB><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
+        case PB_OP_MUL: k_binop<PB_OP_MUL><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
+        case PB_OP_DIV: k_binop<PB_OP_DIV><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
+        default: k_binop<PB_OP_ASSIGN><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
     }
     PB_LAUNCH_CHECK();
     return PB_OK;
@@ -260,15 +286,17 @@ int pb_boxdata_scalar_f64(int op, double* dst, pb_box dst_box, pb_box region, do
     if (bempty(db)) return PB_ERR_BOX;
     r = bempty(r) ? db : intersect(r, db);
     if (bempty(r)) return PB_OK;
-    Region rg = region_of(r);
+    const Region rg = region_of(r);
+    const Walk w = walk_of(rg);
+    const dim3 grid = walk_grid(w, ncomp);
+    const FieldView<double> d = view_of(dst, db, rg);
     cudaStream_t st = (cudaStream_t)stream;
-    int grid = grid_for(bvol(r), 256);
     switch (op) {
-        case PB_OP_ADD: k_scalar<PB_OP_ADD><<<grid, 256, 0, st>>>(dst, db, rg, scalar, ncomp); break;
-        case PB_OP_SUB: k_scalar<PB_OP_SUB><<<grid, 256, 0, st>>>(dst, db, rg, scalar, ncomp); break;
-        case PB_OP_MUL: k_scalar<PB_OP_MUL><<<grid, 256, 0, st>>>(dst, db, rg, scalar, ncomp); break;
-        case PB_OP_DIV: k_scalar<PB_OP_DIV><<<grid, 256, 0, st>>>(dst, db, rg, scalar, ncomp); break;
-        default: k_scalar<PB_OP_ASSIGN><<<grid, 256, 0, st>>>(dst, db, rg, scalar, ncomp); break;
+        case PB_OP_ADD: k_scalar<PB_OP_ADD><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
+        case PB_OP_SUB: k_scalar<PB_OP_SUB><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
+        case PB_OP_MUL: k_scalar<PB_OP_MUL><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
+        case PB_OP_DIV: k_scalar<PB_OP_DIV><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
+        default: k_scalar<PB_OP_ASSIGN><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
     }
     PB_LAUNCH_CHECK();
     return PB_OK;
@@ -285,9 +313,10 @@ int pb_boxdata_copy_f64(const double* src, pb_box src_box, double* dst, pb_box d
     for (int d = 0; d < 3; d++) { dshift.lo[d] = db.lo[d] - sh[d]; dshift.hi[d] = db.hi[d] - sh[d]; }
     r = intersect(r, dshift);
     if (bempty(r)) return PB_OK;
-    Region rg = region_of(r);
-    k_binop<PB_OP_ASSIGN><<<grid_for(bvol(r), 256), 256, 0, (cudaStream_t)stream>>>(dst, db, src, sb, rg, sh[0], sh[1],
-                                                                                   sh[2], ncomp);
+    const Region rg = region_of(r);      // source points; their destinations are shifted
+    const Walk w = walk_of(rg);
+    k_binop<PB_OP_ASSIGN><<<walk_grid(w, ncomp), kWalkThreads, 0, (cudaStream_t)stream>>>(
+        view_of(dst, db, rg, sh), bvol(db), view_of(src, sb, rg), bvol(sb), w, ncomp);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -299,7 +328,10 @@ int pb_forall_axpby_f64(double* out, pb_box out_box, const double* x, pb_box x_b
     Box3 ob = to_box(out_box), xb = to_box(x_box), yb = to_box(y_box);
     Box3 r = intersect(intersect(ob, xb), yb);
     if (bempty(r)) return PB_OK;
-    k_axpby<<<grid_for(bvol(r), 256), 256, 0, (cudaStream_t)stream>>>(out, ob, x, xb, y, yb, region_of(r), a, b);
+    const Region rg = region_of(r);
+    const Walk w = walk_of(rg);
+    k_axpby<<<walk_grid(w, 1), kWalkThreads, 0, (cudaStream_t)stream>>>(view_of(out, ob, rg), view_of(x, xb, rg),
+                                                                        view_of(y, yb, rg), w, a, b);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -313,14 +345,24 @@ int pb_reduce_async_f64(int op, const double* data, pb_box box, pb_box region, d
     RedScratch* s;
     int e = red_scratch(&s);
     if (e != PB_OK) return e;
-    Region rg;
-    if (bempty(r)) { rg.lo[0] = rg.lo[1] = rg.lo[2] = 0; rg.n[0] = rg.n[1] = rg.n[2] = 0; }
+    Region rg;                           // an empty intersection folds nothing: the operation's initial value
+    if (bempty(r)) { rg.lo[0] = b.lo[0]; rg.lo[1] = b.lo[1]; rg.lo[2] = b.lo[2]; rg.n[0] = rg.n[1] = rg.n[2] = 0; }
     else rg = region_of(r);
-    long long total = bempty(r) ? 0 : bvol(r);
-    int grid = (int)((total + kRedThreads - 1) / kRedThreads);
-    if (grid > kRedBlocks) grid = kRedBlocks;
+    const Walk w = walk_of(rg);
+    const int rows = kRedThreads >> w.lx;
+    const long long tiles = (long long)((w.ny + rows - 1) / rows) * ((w.nz + kRedZ - 1) / kRedZ);
+    int grid = tiles < kRedBlocks ? (int)tiles : kRedBlocks;
     if (grid < 1) grid = 1;
-    k_reduce<<<grid, kRedThreads, 0, (cudaStream_t)stream>>>(op, data, b, rg, s->partials, s->ticket, result_dev);
+    const FieldView<const double> f = view_of(data, b, rg);
+    cudaStream_t st = (cudaStream_t)stream;
+    switch (op) {
+        case 0: k_reduce<0><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+        case 1: k_reduce<1><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+        case 2: k_reduce<2><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+        case 3: k_reduce<3><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+        case 4: k_reduce<4><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+        default: k_reduce<5><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
+    }
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -350,8 +392,14 @@ int pb_interp_constant_f64(int ratio, const double* src, pb_box src_box, double*
     rb = intersect(rb, db);
     if (bempty(rb)) return PB_OK;
     // InterpStencil::apply's final stage is "S = scale*Shift::Zeros()", folded like hostApply
-    k_interp_const<<<grid_for(bvol(rb), 256), 256, 0, (cudaStream_t)stream>>>(ratio, src, sb, dst, db, region_of(rb),
-                                                                            overwrite, scale);
+    const Region rg = region_of(rb);
+    const Walk w = walk_of(rg);
+    const dim3 grid = walk_grid(w, 1);
+    const FieldView<double> d = view_of(dst, db, rg);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (ratio == 2) k_interp_const<1><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
+    else if (ratio == 4) k_interp_const<2><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
+    else k_interp_const<-1><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
