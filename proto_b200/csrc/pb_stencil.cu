@@ -18,6 +18,7 @@
 #include "pb_internal.cuh"
 #include "pb_star.cuh"
 #include "pb_stencil_impl.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
@@ -84,39 +85,109 @@ int encode_tmap_3d(CUtensorMap* map, const void* base, int esize, long long Sx, 
 }
 
 // ---- generic table kernel ---------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) k_table(const T* __restrict__ src, T* dst, const TableArgs<T> a)
+// Any table: acc = sum_j c_j * src[first + off_j], first the term of the span's low corner, so every
+// offset is non-negative and, with at most 2^32 source cells, 32 bits wide: a term is then one load
+// from a uniform base plus the thread's 32-bit index, one multiply and one add. A thread takes kWalkZ
+// planes of a point, so a term's coefficient and offset are read once for four cells and four to
+// sixteen loads are in flight (one cell per thread with 64-bit offsets issued about seven
+// instructions per term). Bound by the issue of the terms' loads.
+template <typename T, typename I, int NMAX>
+struct TableKernelArgs {
+    T c[NMAX];
+    I off[NMAX];
+    int n, ncomp, init_zero;
+    long long svol, dvol;      // component strides
+    long long sx, sy, sz;      // source steps per index-box step
+    long long dx, dy, dz;      // destination steps per index-box step
+};
+template <typename T, typename I, int NMAX>
+__global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ src, T* dst,
+                                                        const __grid_constant__ TableKernelArgs<T, I, NMAX> a, Walk w)
 {
-    const long long nx = a.ib.hi[0] - a.ib.lo[0] + 1, ny = a.ib.hi[1] - a.ib.lo[1] + 1,
-                    nz = a.ib.hi[2] - a.ib.lo[2] + 1;
-    const long long total = nx * ny * nz;
-    const long long sSx = a.sb.hi[0] - a.sb.lo[0] + 1, sSy = a.sb.hi[1] - a.sb.lo[1] + 1;
-    const long long dSx = a.db.hi[0] - a.db.lo[0] + 1, dSy = a.db.hi[1] - a.db.lo[1] + 1;
-    const long long svol = sSx * sSy * (a.sb.hi[2] - a.sb.lo[2] + 1);
-    const long long dvol = dSx * dSy * (a.db.hi[2] - a.db.lo[2] + 1);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int p[3];
-        p[0] = a.ib.lo[0] + (int)(i % nx);
-        long long r = i / nx;
-        p[1] = a.ib.lo[1] + (int)(r % ny);
-        p[2] = a.ib.lo[2] + (int)(r / ny);
-        int dp[3];
-        bool inside = true;
-        for (int d = 0; d < 3; d++) {
-            dp[d] = p[d] * a.dr[d] + a.ds[d];
-            inside &= (dp[d] >= a.db.lo[d]) && (dp[d] <= a.db.hi[d]);
-        }
-        if (!inside) continue;
-        const long long di = (dp[0] - a.db.lo[0]) + dSx * ((dp[1] - a.db.lo[1]) + dSy * (long long)(dp[2] - a.db.lo[2]));
-        const long long si = (p[0] * a.sr[0] - a.sb.lo[0]) +
-                             sSx * ((p[1] * a.sr[1] - a.sb.lo[1]) + sSy * (long long)(p[2] * a.sr[2] - a.sb.lo[2]));
-        for (int c = 0; c < a.ncomp; c++) {
-            const T* s = src + c * svol;
-            T* o = dst + c * dvol;
-            T acc = a.init_zero ? T(0) : o[di];
-            for (int j = 0; j < a.n; j++) acc = dadd(acc, dmul(a.c[j], __ldg(s + si + a.off[j])));
-            o[di] = acc;
+    for (int c = blockIdx.z; c < a.ncomp; c += gridDim.z) {
+        const T* sp = src + c * a.svol;
+        T* dp = dst + c * a.dvol;
+        walk_rows(w, [&](int x, int y, int z, int planes) {
+            I at[kWalkZ];
+            T acc[kWalkZ];
+            T* dq = dp + a.dx * x + a.dy * y + a.dz * z;
+            at[0] = (I)(a.sx * x + a.sy * y + a.sz * z);
+#pragma unroll
+            for (int k = 1; k < kWalkZ; k++) at[k] = k < planes ? (I)(at[k - 1] + (I)a.sz) : at[0];
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++) acc[k] = a.init_zero || k >= planes ? T(0) : dq[k * a.dz];
+#pragma unroll 4
+            for (int j = 0; j < a.n; j++) {
+                const T* sj = sp + a.off[j];
+                T v[kWalkZ];
+#pragma unroll
+                for (int k = 0; k < kWalkZ; k++) v[k] = __ldg(sj + at[k]);
+#pragma unroll
+                for (int k = 0; k < kWalkZ; k++) acc[k] = dadd(acc[k], dmul(a.c[j], v[k]));
+            }
+#pragma unroll
+            for (int k = 0; k < kWalkZ; k++)
+                if (k < planes) dq[k * a.dz] = acc[k];
+        });
+    }
+}
+
+// The 19- and 27-point Laplacians (centre, then the other points of the 3^3 cube, z slowest and x
+// fastest; the 19-point table leaves out the corners): a thread walks a column of zd planes with the
+// three planes' nine values in registers, so a cell costs nine loads where the table kernel issues 27.
+// The newest plane's terms come last in the table's order, so its loads overlap the older planes'
+// arithmetic. Bound by FP64 issue (27 multiplies and 27 adds, each rounded: 12 us at 3.95 M cells).
+// Measured (B200, two components of 193 x 161 x 127 FP64 cells) 119 -> 90 us. Below kCubeMin cells the
+// columns are too few to fill the GPU, and the table kernel takes four cells per thread.
+constexpr long long kCubeMin = 1 << 17;
+template <typename T>
+struct CubeArgs {
+    T c[27];                    // by cube position (z+1)*9 + (y+1)*3 + (x+1)
+    int ncomp, init_zero, zd, chunks;
+    long long svol, dvol;
+};
+template <typename T, bool CORNERS>
+__global__ void __launch_bounds__(kWalkThreads, 2) k_cube(FieldView<const T> s, FieldView<T> d,
+                                                          const __grid_constant__ CubeArgs<T> a, Walk w)
+{
+    const int lane = threadIdx.x & ((1 << w.lx) - 1), row = threadIdx.x >> w.lx;
+    const int x = blockIdx.x * (1 << w.lx) + lane, y = blockIdx.y * (kWalkThreads >> w.lx) + row;
+    if (x >= w.nx || y >= w.ny) return;
+    for (int u = blockIdx.z; u < a.chunks * a.ncomp; u += gridDim.z) {
+        const int comp = u / a.chunks, z0 = (u - comp * a.chunks) * a.zd, z1 = min(z0 + a.zd, w.nz);
+        // the cell's column one plane below the chunk
+        const T* q = s.p + comp * a.svol + x + s.sy * y + s.sz * (z0 - 1);
+        T* o = d.p + comp * a.dvol + x + d.sy * y + d.sz * z0;
+        T p0[9], p1[9], p2[9];
+        auto load = [&](T* p) {
+#pragma unroll
+            for (int k = 0; k < 9; k++) p[k] = __ldg(q + (k % 3 - 1) + s.sy * (k / 3 - 1));
+            q += s.sz;
+        };
+        auto cell = [&](const T* lo, const T* mid, const T* hi) {
+            T acc = a.init_zero ? T(0) : *o;
+            acc = dadd(acc, dmul(a.c[13], mid[4]));
+#pragma unroll
+            for (int k = 0; k < 27; k++) {
+                const int dist = (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);
+                if (dist == 0 || (!CORNERS && dist == 3)) continue;
+                const T v = k < 9 ? lo[k % 9] : (k < 18 ? mid[k % 9] : hi[k % 9]);
+                acc = dadd(acc, dmul(a.c[k], v));
+            }
+            *o = acc;
+            o += d.sz;
+        };
+        load(p0);
+        load(p1);
+        for (int z = z0; z < z1; z += 3) {
+            load(p2);
+            cell(p0, p1, p2);
+            if (z + 1 >= z1) break;
+            load(p0);
+            cell(p1, p2, p0);
+            if (z + 2 >= z1) break;
+            load(p1);
+            cell(p2, p0, p1);
         }
     }
 }
@@ -130,6 +201,7 @@ struct pb_stencil {
     int sr[3], dr[3], ds[3];
     int spanLo[3], spanHi[3];
     int shape;               // 0 table, 1 Lap7, 2 Lap13
+    int cube = 0;            // shape 0 on the 3^3 cube in StencilLib's order: 19 or 27 points (0: neither)
 };
 
 namespace pb {
@@ -144,6 +216,26 @@ static bool matches_shape(const pb_stencil* s)
         for (int d = 0; d < 3; d++)
             if (s->offs[3 * j + d] != S::off(j, d)) return false;
     return true;
+}
+
+// 27 (or 19) when the table is StencilLib's 27-point (19-point) one: the centre, then the cube's other
+// points (without its corners) with z slowest and x fastest, ratios 1 and no shift; 0 otherwise
+static int matches_cube(const pb_stencil* s)
+{
+    const int n = (int)s->coefs.size();
+    if (n != 27 && n != 19) return 0;
+    for (int d = 0; d < 3; d++)
+        if (s->sr[d] != 1 || s->dr[d] != 1 || s->ds[d] != 0 || s->offs[d] != 0) return 0;
+    int j = 1;
+    for (int k = 0; k < 27; k++) {
+        const int o[3] = {k % 3 - 1, (k / 3) % 3 - 1, k / 9 - 1};
+        const int dist = (o[0] != 0) + (o[1] != 0) + (o[2] != 0);
+        if (dist == 0 || (n == 19 && dist == 3)) continue;
+        for (int d = 0; d < 3; d++)
+            if (s->offs[3 * j + d] != o[d]) return 0;
+        j++;
+    }
+    return n;
 }
 
 // scale folded into the coefficients as Stencil::hostApply does (Proto_StencilImplem.H:771-779)
@@ -257,6 +349,83 @@ static int resolve_box(const pb_stencil* s, const Box3& sb, const Box3& db, pb_b
     return PB_OK;
 }
 
+// the index-box points whose destination lies in the destination box
+static Box3 clip_to_dst(const pb_stencil* s, Box3 ib, const Box3& db)
+{
+    for (int k = 0; k < 3; k++) {
+        const int lo = ceil_div(db.lo[k] - s->ds[k], s->dr[k]), hi = floor_div(db.hi[k] - s->ds[k], s->dr[k]);
+        if (ib.lo[k] < lo) ib.lo[k] = lo;
+        if (ib.hi[k] > hi) ib.hi[k] = hi;
+    }
+    return ib;
+}
+
+template <typename T, typename I, int NMAX>
+static int launch_table(const pb_stencil* s, const T* src, const Box3& sb, T* dst, const Box3& db, const Box3& ib,
+                        int ncomp, int init_to_zero, T scale, int n, cudaStream_t st)
+{
+    const Region rg = region_of(ib);
+    const Walk w = walk_of(rg);
+    const long long sS[3] = {1, bsize(sb, 0), bsize(sb, 0) * bsize(sb, 1)};
+    const long long dS[3] = {1, bsize(db, 0), bsize(db, 0) * bsize(db, 1)};
+    TableKernelArgs<T, I, NMAX> a;
+    a.n = n;
+    a.ncomp = ncomp;
+    a.init_zero = init_to_zero ? 1 : 0;
+    a.svol = bvol(sb);
+    a.dvol = bvol(db);
+    a.sx = sS[0] * s->sr[0];
+    a.sy = sS[1] * s->sr[1];
+    a.sz = sS[2] * s->sr[2];
+    a.dx = dS[0] * s->dr[0];
+    a.dy = dS[1] * s->dr[1];
+    a.dz = dS[2] * s->dr[2];
+    // first: the span's low corner at the first point (inside the source box when a term is read)
+    for (int d = 0; d < 3; d++) {
+        if (n > 0) src += sS[d] * ((long long)ib.lo[d] * s->sr[d] + s->spanLo[d] - sb.lo[d]);
+        dst += dS[d] * ((long long)ib.lo[d] * s->dr[d] + s->ds[d] - db.lo[d]);
+    }
+    for (int j = 0; j < n; j++) {
+        a.c[j] = fold<T>(s->coefs[j], scale);
+        long long o = 0;
+        for (int d = 0; d < 3; d++) o += sS[d] * (s->offs[3 * j + d] - s->spanLo[d]);
+        a.off[j] = (I)o;
+    }
+    k_table<T, I, NMAX><<<walk_grid(w, ncomp), kWalkThreads, 0, st>>>(src, dst, a, w);
+    PB_LAUNCH_CHECK();
+    return PB_OK;
+}
+
+template <typename T>
+static int launch_cube(const pb_stencil* s, const T* src, const Box3& sb, T* dst, const Box3& db, const Box3& ib,
+                       int ncomp, int init_to_zero, T scale, cudaStream_t st)
+{
+    const Region rg = region_of(ib);
+    const Walk w = walk_of(rg);
+    CubeArgs<T> a{};
+    a.ncomp = ncomp;
+    a.init_zero = init_to_zero ? 1 : 0;
+    a.svol = bvol(sb);
+    a.dvol = bvol(db);
+    for (int j = 0; j < (int)s->coefs.size(); j++)
+        a.c[(s->offs[3 * j + 2] + 1) * 9 + (s->offs[3 * j + 1] + 1) * 3 + s->offs[3 * j] + 1] = fold<T>(s->coefs[j], scale);
+    const int rows = kWalkThreads >> w.lx, gx = (w.nx + (1 << w.lx) - 1) >> w.lx, gy = (w.ny + rows - 1) / rows;
+    // chunks of z: each starts with two planes of loads beyond its own, so as deep as still leaves
+    // about eight blocks per SM in all
+    a.zd = w.nz;
+    const long long want = 8LL * cached_sm_count();
+    while (a.zd > 8 && (long long)gx * gy * ((w.nz + a.zd - 1) / a.zd) * ncomp < want) a.zd = (a.zd + 1) / 2;
+    a.chunks = (w.nz + a.zd - 1) / a.zd;
+    const long long gz = (long long)a.chunks * ncomp;
+    const dim3 grid(gx, gy, (unsigned)(gz < 65535 ? gz : 65535));
+    const FieldView<const T> sv = view_of(src, sb, rg);
+    const FieldView<T> dv = view_of(dst, db, rg);
+    if (s->cube == 27) k_cube<T, true><<<grid, kWalkThreads, 0, st>>>(sv, dv, a, w);
+    else k_cube<T, false><<<grid, kWalkThreads, 0, st>>>(sv, dv, a, w);
+    PB_LAUNCH_CHECK();
+    return PB_OK;
+}
+
 template <typename T>
 static int apply_impl(const pb_stencil* s, const T* src, pb_box src_box, T* dst, pb_box dst_box, pb_box box,
                       int ncomp, int init_to_zero, T scale, cudaStream_t st)
@@ -270,16 +439,9 @@ static int apply_impl(const pb_stencil* s, const T* src, pb_box src_box, T* dst,
     if (scale == T(0)) {
         // the reference zeroes the destination for "|=" and does nothing else
         if (!init_to_zero) return PB_OK;
-        TableArgs<T> a;
-        memset(&a, 0, sizeof(a));
-        a.n = 0;
-        a.ncomp = ncomp;
-        a.init_zero = 1;
-        a.sb = sb; a.db = db; a.ib = ib;
-        for (int k = 0; k < 3; k++) { a.sr[k] = s->sr[k]; a.dr[k] = s->dr[k]; a.ds[k] = s->ds[k]; }
-        k_table<T><<<grid_for(bvol(ib), 256), 256, 0, st>>>(src, dst, a);
-        PB_LAUNCH_CHECK();
-        return PB_OK;
+        ib = clip_to_dst(s, ib, db);
+        if (bempty(ib)) return PB_OK;
+        return launch_table<T, unsigned, 32>(s, src, sb, dst, db, ib, ncomp, 1, scale, 0, st);
     }
     const long long svol = bvol(sb), dvol = bvol(db);
     if (s->shape == 1 || s->shape == 2) {
@@ -299,22 +461,15 @@ static int apply_impl(const pb_stencil* s, const T* src, pb_box src_box, T* dst,
         }
         return PB_OK;
     }
-    int n = (int)s->coefs.size();
+    const int n = (int)s->coefs.size();
     if (n > kMaxTerms) return PB_ERR_UNSUPPORTED;
-    TableArgs<T> a;
-    a.n = n;
-    a.ncomp = ncomp;
-    a.init_zero = init_to_zero ? 1 : 0;
-    a.sb = sb; a.db = db; a.ib = ib;
-    for (int k = 0; k < 3; k++) { a.sr[k] = s->sr[k]; a.dr[k] = s->dr[k]; a.ds[k] = s->ds[k]; }
-    const long long sSx = bsize(sb, 0), sSxy = bsize(sb, 0) * bsize(sb, 1);
-    for (int j = 0; j < n; j++) {
-        a.c[j] = fold<T>(s->coefs[j], scale);
-        a.off[j] = s->offs[3 * j] + sSx * s->offs[3 * j + 1] + sSxy * s->offs[3 * j + 2];
-    }
-    k_table<T><<<grid_for(bvol(ib), 256), 256, 0, st>>>(src, dst, a);
-    PB_LAUNCH_CHECK();
-    return PB_OK;
+    ib = clip_to_dst(s, ib, db);
+    if (bempty(ib)) return PB_OK;
+    if (s->cube && bvol(ib) >= kCubeMin && (bsize(ib, 1) + 7) / 8 <= 65535)
+        return launch_cube<T>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, st);
+    if (svol > 0xffffffffLL) return launch_table<T, long long, kMaxTerms>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
+    if (n <= 32) return launch_table<T, unsigned, 32>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
+    return launch_table<T, unsigned, kMaxTerms>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
 }
 
 } // namespace pb
@@ -388,6 +543,7 @@ int pb_stencil_create(const double* coefs, const int* offsets, int nterms, const
             if (j == 0 || v > s->spanHi[d]) s->spanHi[d] = v;
         }
     s->shape = matches_shape<ShapeLap7>(s) ? 1 : matches_shape<ShapeLap13>(s) ? 2 : 0;
+    s->cube = matches_cube(s);
     *out = s;
     return PB_OK;
 }

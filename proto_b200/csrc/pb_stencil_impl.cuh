@@ -9,15 +9,6 @@ namespace pb {
 
 constexpr int kMaxTerms = 256;
 
-template <typename T>
-struct TableArgs {
-    T c[kMaxTerms];
-    long long off[kMaxTerms];
-    int n, ncomp, init_zero;
-    Box3 sb, db, ib;
-    int sr[3], dr[3], ds[3];
-};
-
 // Launch-shape knobs for the star kernels (set by the autotuner; defaults are heuristic).
 struct StarTune {
     enum Mode { AUTO = 0, TMA = 1, SIMPLE = 2 };
