@@ -28,19 +28,49 @@ struct MotionItem {
     int sh[3];                 // source point = destination point - sh
 };
 
-__global__ void __launch_bounds__(256) k_exchange(double* slab, const MotionItem* __restrict__ items, int ncomp)
+// A unit of exchange work: up to kUnitCells consecutive cells (x fastest) of one item's region, the
+// first at region coordinates (x, y, z). A region is 8 cells at a corner and thousands on a face, so
+// a warp per unit balances them; each lane keeps kUnitCells / 32 loads in flight. Bound by the ghost
+// cells' bytes (the x faces move 16-byte pieces of 32-byte sectors) and memory latency. Measured (B200,
+// 1498 items of 2 ghost cells): 29.8 -> 12.4 us against one block per item with one cell per thread and
+// 64-bit divisions.
+constexpr int kUnitCells = 256;
+struct ExchangeUnit {
+    int item;
+    int x, y, z;
+    int count;
+};
+
+__global__ void __launch_bounds__(256) k_exchange(double* slab, const MotionItem* __restrict__ items,
+                                                  const ExchangeUnit* __restrict__ units, int nunits, int ncomp)
 {
-    const MotionItem it = items[blockIdx.x];
-    const long long total = (long long)it.rn[0] * it.rn[1] * it.rn[2];
-    for (long long i = threadIdx.x; i < total; i += blockDim.x) {
-        int x = it.rlo[0] + (int)(i % it.rn[0]);
-        long long q = i / it.rn[0];
-        int y = it.rlo[1] + (int)(q % it.rn[1]);
-        int z = it.rlo[2] + (int)(q / it.rn[1]);
-        long long di = (x - it.dlo[0]) + (long long)it.dS[0] * ((y - it.dlo[1]) + (long long)it.dS[1] * (z - it.dlo[2]));
-        int sx = x - it.sh[0], sy = y - it.sh[1], sz = z - it.sh[2];
-        long long si = (sx - it.slo[0]) + (long long)it.sS[0] * ((sy - it.slo[1]) + (long long)it.sS[1] * (sz - it.slo[2]));
-        for (int c = 0; c < ncomp; c++) slab[it.dOff + c * it.dvol + di] = slab[it.sOff + c * it.svol + si];
+    const int u = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (u >= nunits) return;
+    const ExchangeUnit un = units[u];
+    const MotionItem& it = items[un.item];
+    constexpr int K = kUnitCells / 32;
+    const unsigned nx = it.rn[0], ny = it.rn[1];
+    const long long dSx = it.dS[0], dSxy = dSx * it.dS[1], sSx = it.sS[0], sSxy = sSx * it.sS[1];
+    // region coordinate (0, 0, 0) in the destination and in the source
+    double* d0 = slab + it.dOff + (it.rlo[0] - it.dlo[0]) + dSx * (it.rlo[1] - it.dlo[1]) + dSxy * (it.rlo[2] - it.dlo[2]);
+    const double* s0 = slab + it.sOff + (it.rlo[0] - it.sh[0] - it.slo[0]) + sSx * (it.rlo[1] - it.sh[1] - it.slo[1]) +
+                       sSxy * (it.rlo[2] - it.sh[2] - it.slo[2]);
+    long long di[K], si[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const unsigned px = un.x + lane + 32 * k, qy = px / nx, py = un.y + qy, qz = py / ny;
+        const long long x = px - qy * nx, y = py - qz * ny, z = un.z + qz;
+        di[k] = x + dSx * y + dSxy * z;
+        si[k] = x + sSx * y + sSxy * z;
+    }
+    for (int c = 0; c < ncomp; c++) {
+        double v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+            if (lane + 32 * k < un.count) v[k] = s0[c * it.svol + si[k]];
+#pragma unroll
+        for (int k = 0; k < K; k++)
+            if (lane + 32 * k < un.count) d0[c * it.dvol + di[k]] = v[k];
     }
 }
 
@@ -516,6 +546,8 @@ struct pb_level {
     long long slab_elems;
     std::vector<pb::MotionItem> items;
     pb::MotionItem* d_items = nullptr;
+    std::vector<pb::ExchangeUnit> units;       // the items' regions in warp-sized pieces
+    pb::ExchangeUnit* d_units = nullptr;
     std::vector<pb::PatchTile> tiles;          // one cell per thread
     pb::PatchTile* d_tiles = nullptr;
     std::vector<pb::PatchTile> tiles2;         // two x cells per thread (fused halo-2 steps, pair_ok)
@@ -583,6 +615,26 @@ static void build_items(pb_level* lv)
                     }
         }
     }
+}
+
+static void build_units(pb_level* lv)
+{
+    for (int i = 0; i < (int)lv->items.size(); i++) {
+        const MotionItem& m = lv->items[i];
+        const long long nx = m.rn[0], ny = m.rn[1], vol = nx * ny * m.rn[2];
+        for (long long f = 0; f < vol; f += kUnitCells)
+            lv->units.push_back(ExchangeUnit{i, (int)(f % nx), (int)(f / nx % ny), (int)(f / (nx * ny)),
+                                             (int)std::min<long long>(kUnitCells, vol - f)});
+    }
+}
+
+static int launch_exchange(const pb_level* lv, double* slab, cudaStream_t st)
+{
+    const int nu = (int)lv->units.size();
+    if (nu == 0) return PB_OK;
+    k_exchange<<<(nu + 7) / 8, 256, 0, st>>>(slab, lv->d_items, lv->d_units, nu, lv->ncomp);
+    PB_LAUNCH_CHECK();
+    return PB_OK;
 }
 
 static std::pair<int, int> tile_shape(const pb_level* lv, int nx, int xv = 1)
@@ -865,6 +917,7 @@ int pb_level_create(const pb_box* patches, int npatch, const int ghost[3], pb_bo
     }
     lv->slab_elems = off;
     build_items(lv);
+    build_units(lv);
     detect_tensor(lv);
     lv->pair_ok = lv->tensor && ncomp == 1 && ghost[0] % 2 == 0;
     for (const Box3& b : lv->patches) lv->pair_ok = lv->pair_ok && bsize(b, 0) % 2 == 0;
@@ -874,14 +927,19 @@ int pb_level_create(const pb_box* patches, int npatch, const int ghost[3], pb_bo
     if (!lv->items.empty()) {
         if (cudaMalloc(&lv->d_items, lv->items.size() * sizeof(MotionItem)) != cudaSuccess ||
             cudaMemcpy(lv->d_items, lv->items.data(), lv->items.size() * sizeof(MotionItem), cudaMemcpyHostToDevice) !=
+                cudaSuccess ||
+            cudaMalloc(&lv->d_units, lv->units.size() * sizeof(ExchangeUnit)) != cudaSuccess ||
+            cudaMemcpy(lv->d_units, lv->units.data(), lv->units.size() * sizeof(ExchangeUnit), cudaMemcpyHostToDevice) !=
                 cudaSuccess) {
             cudaFree(lv->d_items);
+            cudaFree(lv->d_units);
             delete lv;
             return PB_ERR_CUDA;
         }
     }
     if (upload_tiles(lv) != PB_OK || upload_tiles(lv, 2) != PB_OK) {
         cudaFree(lv->d_items);
+        cudaFree(lv->d_units);
         cudaFree(lv->d_tiles);
         delete lv;
         return PB_ERR_CUDA;
@@ -895,6 +953,7 @@ int pb_level_destroy(pb_level* lv)
     if (!lv) return PB_OK;
     drop_graph(lv);
     cudaFree(lv->d_items);
+    cudaFree(lv->d_units);
     cudaFree(lv->d_tiles);
     cudaFree(lv->d_tiles2);
     delete lv;
@@ -913,10 +972,7 @@ int pb_level_layout(const pb_level* lv, long long* offsets, long long* slab_elem
 int pb_level_exchange_f64(const pb_level* lv, double* slab, void* stream)
 {
     if (!lv || !slab) return PB_ERR_ARG;
-    if (lv->items.empty()) return PB_OK;
-    k_exchange<<<(unsigned)lv->items.size(), 256, 0, (cudaStream_t)stream>>>(slab, lv->d_items, lv->ncomp);
-    PB_LAUNCH_CHECK();
-    return PB_OK;
+    return launch_exchange(lv, slab, (cudaStream_t)stream);
 }
 
 int pb_level_stencil_f64(const pb_level* lv, const pb_stencil* s, int epilogue, const double* u_slab, double* out_slab,
@@ -959,10 +1015,7 @@ int pb_level_steps_f64(pb_level* lv, const pb_stencil* s, int epilogue, double* 
         double* a_ = u_slab;
         double* b_ = tmp_slab;
         for (int k = 0; k < steps && e == PB_OK; k++) {
-            if (!lv->tensor && !lv->items.empty()) {
-                k_exchange<<<(unsigned)lv->items.size(), 256, 0, cs>>>(a_, lv->d_items, lv->ncomp);
-                if (cudaGetLastError() != cudaSuccess) e = PB_ERR_CUDA;
-            }
+            if (!lv->tensor) e = launch_exchange(lv, a_, cs);
             if (e == PB_OK) e = launch_level_star(lv, shape, a_, b_, cf, a, epilogue == PB_EPI_EULER, cs, lv->tensor);
             std::swap(a_, b_);
         }
