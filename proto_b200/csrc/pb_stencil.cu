@@ -133,13 +133,16 @@ __global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ sr
 }
 
 // The 19- and 27-point Laplacians (centre, then the other points of the 3^3 cube, z slowest and x
-// fastest; the 19-point table leaves out the corners): a thread walks a column of zd planes with the
-// three planes' nine values in registers, so a cell costs nine loads where the table kernel issues 27.
-// The newest plane's terms come last in the table's order, so its loads overlap the older planes'
-// arithmetic. Bound by FP64 issue (27 multiplies and 27 adds, each rounded: 12 us at 3.95 M cells).
-// Measured (B200, two components of 193 x 161 x 127 FP64 cells) 119 -> 90 us. Below kCubeMin cells the
-// columns are too few to fill the GPU, and the table kernel takes four cells per thread.
+// fastest; the 19-point table leaves out the corners): a thread walks a column of zd planes, reading each
+// plane's nine values once (the table kernel issues 27 loads a cell). In the table's order the terms of
+// the plane above come last, so a cell's sum is carried over from the step that completes its lower two
+// planes, and only the previous, the current and the next plane (on its way, a whole step early) are in
+// registers. Bound by FP64 issue (27 multiplies and 27 adds, each rounded: 12 us at 3.95 M cells) and
+// load latency. Measured (B200, two components of 193 x 161 x 127 FP64 cells): 68 us a component one cell
+// per thread, 43 with the three planes held, 33 with the next plane loaded a step early. Below kCubeMin cells the columns are too few to fill the GPU, and the table kernel takes
+// four cells per thread.
 constexpr long long kCubeMin = 1 << 17;
+constexpr int kCubeThreads = 128, kCubePerSm = 5;
 template <typename T>
 struct CubeArgs {
     T c[27];                    // by cube position (z+1)*9 + (y+1)*3 + (x+1)
@@ -147,47 +150,54 @@ struct CubeArgs {
     long long svol, dvol;
 };
 template <typename T, bool CORNERS>
-__global__ void __launch_bounds__(kWalkThreads, 2) k_cube(FieldView<const T> s, FieldView<T> d,
-                                                          const __grid_constant__ CubeArgs<T> a, Walk w)
+__global__ void __launch_bounds__(kCubeThreads, kCubePerSm) k_cube(FieldView<const T> s, FieldView<T> d,
+                                                                   const __grid_constant__ CubeArgs<T> a, Walk w)
 {
     const int lane = threadIdx.x & ((1 << w.lx) - 1), row = threadIdx.x >> w.lx;
-    const int x = blockIdx.x * (1 << w.lx) + lane, y = blockIdx.y * (kWalkThreads >> w.lx) + row;
+    const int x = blockIdx.x * (1 << w.lx) + lane, y = blockIdx.y * (kCubeThreads >> w.lx) + row;
     if (x >= w.nx || y >= w.ny) return;
     for (int u = blockIdx.z; u < a.chunks * a.ncomp; u += gridDim.z) {
         const int comp = u / a.chunks, z0 = (u - comp * a.chunks) * a.zd, z1 = min(z0 + a.zd, w.nz);
-        // the cell's column one plane below the chunk
-        const T* q = s.p + comp * a.svol + x + s.sy * y + s.sz * (z0 - 1);
-        T* o = d.p + comp * a.dvol + x + d.sy * y + d.sz * z0;
-        T p0[9], p1[9], p2[9];
+        const T* q = s.p + comp * a.svol + x + s.sy * y + s.sz * (z0 - 1);   // the next plane to load
+        T* o = d.p + comp * a.dvol + x + d.sy * y + d.sz * z0;               // the next cell to start
         auto load = [&](T* p) {
 #pragma unroll
             for (int k = 0; k < 9; k++) p[k] = __ldg(q + (k % 3 - 1) + s.sy * (k / 3 - 1));
             q += s.sz;
         };
-        auto cell = [&](const T* lo, const T* mid, const T* hi) {
-            T acc = a.init_zero ? T(0) : *o;
-            acc = dadd(acc, dmul(a.c[13], mid[4]));
-#pragma unroll
-            for (int k = 0; k < 27; k++) {
-                const int dist = (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);
-                if (dist == 0 || (!CORNERS && dist == 3)) continue;
-                const T v = k < 9 ? lo[k % 9] : (k < 18 ? mid[k % 9] : hi[k % 9]);
-                acc = dadd(acc, dmul(a.c[k], v));
-            }
-            *o = acc;
-            o += d.sz;
+        auto term = [&](T& acc, int k, T v) {
+            const int dist = (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);
+            if (dist != 0 && (CORNERS || dist != 3)) acc = dadd(acc, dmul(a.c[k], v));
         };
+        T acc = T(0);
+        // plane z of the chunk in cur, z - 1 in prev, z + 1 on its way into next: completes cell z - 1
+        // (its upper plane), then starts cell z
+        auto step = [&](const T* prev, const T* cur, T* next, int z) {
+            if (z < z1) load(next);
+            if (z > z0) {
+#pragma unroll
+                for (int k = 18; k < 27; k++) term(acc, k, cur[k - 18]);
+                *(o - d.sz) = acc;
+            }
+            if (z < z1) {
+                acc = a.init_zero ? T(0) : *o;
+                acc = dadd(acc, dmul(a.c[13], cur[4]));
+#pragma unroll
+                for (int k = 0; k < 9; k++) term(acc, k, prev[k]);
+#pragma unroll
+                for (int k = 9; k < 18; k++) term(acc, k, cur[k - 9]);
+                o += d.sz;
+            }
+        };
+        T p0[9], p1[9], p2[9];
         load(p0);
         load(p1);
-        for (int z = z0; z < z1; z += 3) {
-            load(p2);
-            cell(p0, p1, p2);
-            if (z + 1 >= z1) break;
-            load(p0);
-            cell(p1, p2, p0);
-            if (z + 2 >= z1) break;
-            load(p1);
-            cell(p2, p0, p1);
+        for (int z = z0; z <= z1; z += 3) {
+            step(p0, p1, p2, z);
+            if (z + 1 > z1) break;
+            step(p1, p2, p0, z + 1);
+            if (z + 2 > z1) break;
+            step(p2, p0, p1, z + 2);
         }
     }
 }
@@ -409,19 +419,26 @@ static int launch_cube(const pb_stencil* s, const T* src, const Box3& sb, T* dst
     a.dvol = bvol(db);
     for (int j = 0; j < (int)s->coefs.size(); j++)
         a.c[(s->offs[3 * j + 2] + 1) * 9 + (s->offs[3 * j + 1] + 1) * 3 + s->offs[3 * j] + 1] = fold<T>(s->coefs[j], scale);
-    const int rows = kWalkThreads >> w.lx, gx = (w.nx + (1 << w.lx) - 1) >> w.lx, gy = (w.ny + rows - 1) / rows;
-    // chunks of z: each starts with two planes of loads beyond its own, so as deep as still leaves
-    // about eight blocks per SM in all
-    a.zd = w.nz;
-    const long long want = 8LL * cached_sm_count();
-    while (a.zd > 8 && (long long)gx * gy * ((w.nz + a.zd - 1) / a.zd) * ncomp < want) a.zd = (a.zd + 1) / 2;
+    const int rows = kCubeThreads >> w.lx, gx = (w.nx + (1 << w.lx) - 1) >> w.lx, gy = (w.ny + rows - 1) / rows;
+    // the z chunk that makes waves of resident blocks x (planes + 2) smallest: a chunk starts with two
+    // planes of loads beyond its own
+    const long long slots = (long long)kCubePerSm * cached_sm_count();
+    long long best = -1;
+    for (int zd = 4; zd < w.nz + 4; zd += zd < 64 ? 4 : 16) {
+        const long long blocks = (long long)gx * gy * ((w.nz + zd - 1) / zd) * ncomp;
+        const long long cost = (blocks + slots - 1) / slots * (zd + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            a.zd = zd;
+        }
+    }
     a.chunks = (w.nz + a.zd - 1) / a.zd;
     const long long gz = (long long)a.chunks * ncomp;
     const dim3 grid(gx, gy, (unsigned)(gz < 65535 ? gz : 65535));
     const FieldView<const T> sv = view_of(src, sb, rg);
     const FieldView<T> dv = view_of(dst, db, rg);
-    if (s->cube == 27) k_cube<T, true><<<grid, kWalkThreads, 0, st>>>(sv, dv, a, w);
-    else k_cube<T, false><<<grid, kWalkThreads, 0, st>>>(sv, dv, a, w);
+    if (s->cube == 27) k_cube<T, true><<<grid, kCubeThreads, 0, st>>>(sv, dv, a, w);
+    else k_cube<T, false><<<grid, kCubeThreads, 0, st>>>(sv, dv, a, w);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -465,7 +482,7 @@ static int apply_impl(const pb_stencil* s, const T* src, pb_box src_box, T* dst,
     if (n > kMaxTerms) return PB_ERR_UNSUPPORTED;
     ib = clip_to_dst(s, ib, db);
     if (bempty(ib)) return PB_OK;
-    if (s->cube && bvol(ib) >= kCubeMin && (bsize(ib, 1) + 7) / 8 <= 65535)
+    if (s->cube && bvol(ib) >= kCubeMin && (bsize(ib, 1) + 3) / 4 <= 65535)
         return launch_cube<T>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, st);
     if (svol > 0xffffffffLL) return launch_table<T, long long, kMaxTerms>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
     if (n <= 32) return launch_table<T, unsigned, 32>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
