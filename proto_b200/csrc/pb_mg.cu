@@ -179,8 +179,21 @@ static int launch_relax(pb_mg* mg, MGLevel<T>& L, bool first, cudaStream_t st)
 {
     const RelaxCoef<T> k = relax_coef(mg, L);
     if (first) {
-        const long long total = (long long)L.n * L.n * L.n;
-        k_relax_first<T><<<grid_for(total, 256), 256, 0, st>>>(L.rhs, L.alpha, L.phi[1 - L.cur], k);
+        const Walk w = walk_cube(L.n);
+        k_relax_first<T><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(L.rhs, L.alpha, L.phi[1 - L.cur], k, w);
+        PB_LAUNCH_CHECK();
+    } else if (L.n > 1 && L.n < kMarchEdge) {
+        // lanes along x: the smallest power of two that holds a row, 8 to 32; z chunks for two blocks per SM
+        int lx = 5, zd = 8;
+        while (lx > 3 && (1 << (lx - 1)) >= L.n) lx--;
+        const int rows = 2 * (256 >> lx), gx = (L.n + (1 << lx) - 1) >> lx, gy = (L.n + rows - 1) / rows;
+        while (zd > 1 && (long long)gx * gy * ((L.n + zd - 1) / zd) < 2LL * cached_sm_count()) zd /= 2;
+        const Coefs<T> c = lap7_coefs<T>(is_helm(mg) ? L.hsqinv : mg->p.omega / 6.0);
+        const dim3 grid(gx, gy, (L.n + zd - 1) / zd);
+        if (is_helm(mg))
+            k_relax_march<T, true><<<grid, 256, 0, st>>>(L.phi[L.cur], L.phi[1 - L.cur], L.rhs, L.alpha, k, c.c[0], c.c[1], lx, zd);
+        else
+            k_relax_march<T, false><<<grid, 256, 0, st>>>(L.phi[L.cur], L.phi[1 - L.cur], L.rhs, L.alpha, k, c.c[0], c.c[1], lx, zd);
         PB_LAUNCH_CHECK();
     } else {
         EpiRelax<T> epi;
@@ -865,15 +878,16 @@ int pb_mg_solve(pb_mg* mg, const double* rhs, double* phi, int* iters, double* h
     const long long n3 = (long long)n * n * n;
     int e;
     MGLevel<double>* T = mixed ? nullptr : &mg->lv.back();
+    const Walk wg = walk_cube(n + 2);
     if (mixed) {
         PB_CUDA(cudaMemcpyAsync(mg->f64, rhs, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
-        k_pack_in<double><<<grid_for(n3, 256), 256, 0, st>>>(phi, mg->u64, n, grown_pitch<double>(n));
+        k_pack_in<double><<<walk_grid(wg, 1), kWalkThreads, 0, st>>>(phi, mg->u64, n, grown_pitch<double>(n), wg);
         PB_LAUNCH_CHECK();
         if ((e = launch_res64(mg, st)) != PB_OK) return e;
     } else {
         PB_CUDA(cudaMemcpyAsync(T->rhs, rhs, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
         T->cur = 0;
-        k_pack_in<double><<<grid_for(n3, 256), 256, 0, st>>>(phi, T->phi[0], n, T->sx);
+        k_pack_in<double><<<walk_grid(wg, 1), kWalkThreads, 0, st>>>(phi, T->phi[0], n, T->sx, wg);
         PB_LAUNCH_CHECK();
         e = fuse_norm(mg) ? launch_relax_norm(mg, *T, st) : launch_resnorm(mg, *T, st);
         if (e != PB_OK) return e;
@@ -921,7 +935,8 @@ int pb_mg_solve(pb_mg* mg, const double* rhs, double* phi, int* iters, double* h
         if (r < mg->p.tol * r0) break;
     }
     const double* src = mixed ? mg->u64 : T->phi[T->cur];
-    k_pack_out<double><<<grid_for(n3, 256), 256, 0, st>>>(src, phi, n, grown_pitch<double>(n));
+    const Walk wv = walk_cube(n);
+    k_pack_out<double><<<walk_grid(wv, 1), kWalkThreads, 0, st>>>(src, phi, n, grown_pitch<double>(n), wv);
     PB_LAUNCH_CHECK();
     PB_CUDA(cudaStreamSynchronize(st));
     if (read_error_mg() > 0 || read_error_stencil() > 0) return PB_ERR_DEVICE;

@@ -8,6 +8,7 @@
 
 #include "pb_internal.cuh"
 #include "pb_star.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
@@ -343,18 +344,87 @@ struct EpiRes64 {
 
 // first sweep from phi == 0 (every read of phi would return +0.0)
 template <typename T>
-__global__ void __launch_bounds__(256) k_relax_first(const T* __restrict__ rhs, const T* __restrict__ alpha, T* out,
-                                                     RelaxCoef<T> k)
+__global__ void __launch_bounds__(kWalkThreads) k_relax_first(const T* __restrict__ rhs, const T* __restrict__ alpha,
+                                                              T* out, RelaxCoef<T> k, Walk w)
 {
     const int n = k.n;
-    const long long total = (long long)n * n * n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = (int)(i % n);
-        long long q = i / n;
-        int y = (int)(q % n), z = (int)(q / n);
-        const T al = k.helm ? alpha[i] : T(0);
-        store_periodic(out, n, k.sx, x, y, z, relax_value(k, T(0), T(0), rhs[i], al));
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        const long long i = x + (long long)n * (y + (long long)n * z), n2 = (long long)n * n;
+        T rho[kWalkZ], al[kWalkZ];
+#pragma unroll
+        for (int j = 0; j < kWalkZ; j++)
+            if (j < planes) {
+                rho[j] = __ldg(rhs + i + j * n2);
+                al[j] = k.helm ? __ldg(alpha + i + j * n2) : T(0);
+            }
+#pragma unroll
+        for (int j = 0; j < kWalkZ; j++)
+            if (j < planes) store_periodic(out, n, k.sx, x, y, z + j, relax_value(k, T(0), T(0), rho[j], al[j]));
+    });
+}
+
+// One sweep of a level too small for the staged kernels (below kMarchEdge), as a march: a thread takes
+// two rows of one x and zd planes, keeps the rows' values at three planes in registers and reads the
+// x neighbours and the two rows beyond from L1-resident rows, so a cell costs four loads and no 64-bit
+// division, and a plane's loads are all in flight together. These sweeps take as long as a launch and
+// two memory latencies; the staged kernel's ring fill and the one-cell kernel's index arithmetic came on
+// top. Same arithmetic as EpiRelax (taps in the Laplacian's order, relax_value).
+constexpr int kMarchEdge = 128;
+template <typename T, bool HELM>
+__global__ void __launch_bounds__(256) k_relax_march(const T* __restrict__ phi, T* out, const T* __restrict__ rhs,
+                                                     const T* __restrict__ alpha, RelaxCoef<T> k, T c0, T cn, int lx,
+                                                     int zd)
+{
+    const int n = k.n, sx = k.sx;
+    const int x = blockIdx.x * (1 << lx) + (threadIdx.x & ((1 << lx) - 1));
+    const int y = 2 * (blockIdx.y * (256 >> lx) + (threadIdx.x >> lx));
+    if (x >= n || y >= n) return;
+    const int z0 = blockIdx.z * zd, z1 = min(z0 + zd, n);
+    const bool two = y + 1 < n;                                  // an odd edge leaves the last row alone
+    const long long Sz = (long long)sx * (n + 2);
+    const T* q = phi + grown_index<T>(n, sx, x, y, z0);
+    const int s2 = two ? 2 * sx : sx;                            // row y + 2 (row y + 1 is the ghost row otherwise)
+    T* o = out + grown_index<T>(n, sx, x, y, z0);
+    long long i = x + (long long)n * (y + (long long)n * z0);
+    const int exy = edge_code(x, n) | edge_code(y, n) | (two ? edge_code(y + 1, n) : 0);
+    T zm[2] = {q[-Sz], q[sx - Sz]}, zc[2] = {q[0], q[sx]};
+    for (int z = z0; z < z1; z++) {
+        const int ez = edge_code(z, n);
+        const T zp[2] = {q[Sz], q[Sz + sx]};
+        const T xm[2] = {q[-1], q[sx - 1]}, xp[2] = {q[1], q[sx + 1]};
+        const T yb = q[-sx], yt = q[s2];
+        T rho[2], al[2] = {T(0), T(0)};
+        rho[0] = __ldg(rhs + i);
+        rho[1] = two ? __ldg(rhs + i + n) : T(0);
+        if constexpr (HELM) {
+            al[0] = __ldg(alpha + i);
+            al[1] = two ? __ldg(alpha + i + n) : T(1);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            // 0, +x, -x, +y, -y, +z, -z
+            T acc = T(0);
+            acc = dmadd(acc, c0, zc[r]);
+            acc = dmadd(acc, cn, xp[r]);
+            acc = dmadd(acc, cn, xm[r]);
+            acc = dmadd(acc, cn, r == 0 ? zc[1] : yt);
+            acc = dmadd(acc, cn, r == 0 ? yb : zc[0]);
+            acc = dmadd(acc, cn, zp[r]);
+            acc = dmadd(acc, cn, zm[r]);
+            const T v = relax_value(k, acc, zc[r], rho[r], al[r]);
+            if (r == 0 || two) {
+                if (exy | ez) store_with_images(out, n, sx, o + r * sx, edge_code(x, n), edge_code(y + r, n), ez, v);
+                else o[r * sx] = v;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            zm[r] = zc[r];
+            zc[r] = zp[r];
+        }
+        q += Sz;
+        o += Sz;
+        i += (long long)n * n;
     }
 }
 
@@ -721,28 +791,36 @@ __global__ void __launch_bounds__(256) k_prolong(T* phi, const T* __restrict__ d
 }
 static inline dim3 prolong_grid(int nf) { return dim3((nf + 63) / 64, (nf / 2 + 7) / 8, nf / 2); }
 
-// n^3 <-> grown layout with periodic ghost images
+// n^3 <-> grown layout with periodic ghost images. Into the grown layout every grown cell reads the valid
+// cell it is or images, so stores are coalesced and no image is written apart.
 template <typename T>
-__global__ void __launch_bounds__(256) k_pack_in(const T* __restrict__ src, T* out, int n, int sx)
+__global__ void __launch_bounds__(kWalkThreads) k_pack_in(const T* __restrict__ src, T* out, int n, int sx, Walk w)
 {
-    const long long total = (long long)n * n * n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = (int)(i % n);
-        long long q = i / n;
-        store_periodic(out, n, sx, x, (int)(q % n), (int)(q / n), src[i]);
-    }
+    const long long Sz = (long long)sx * (n + 2), n2 = (long long)n * n;
+    auto wrap = [&](int c) { return c == 0 ? n - 1 : (c > n ? 0 : c - 1); };   // grown coordinate -> valid cell
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        const T* q = src + wrap(x) + (long long)n * wrap(y);
+        T v[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) v[k] = __ldg(q + n2 * wrap(z + k));
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) out[x + (long long)sx * y + Sz * (z + k)] = v[k];
+    });
 }
 template <typename T>
-__global__ void __launch_bounds__(256) k_pack_out(const T* __restrict__ g, T* dst, int n, int sx)
+__global__ void __launch_bounds__(kWalkThreads) k_pack_out(const T* __restrict__ g, T* dst, int n, int sx, Walk w)
 {
-    const long long total = (long long)n * n * n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        int x = (int)(i % n);
-        long long q = i / n;
-        dst[i] = g[grown_index<T>(n, sx, x, (int)(q % n), (int)(q / n))];
-    }
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        T v[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) v[k] = __ldg(g + grown_index<T>(n, sx, x, y, z + k));
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) dst[x + (long long)n * (y + (long long)n * (z + k))] = v[k];
+    });
 }
 
 // AvgDown(2) of a plain n^3 field (coarse-level alpha)
