@@ -113,12 +113,12 @@ __global__ void __launch_bounds__(2 * NXT + 32, relax2_min_blocks(2 * NXT + 32))
     using SH = Relax2Shape<NXT, PV, RG>;
     constexpr int N = SH::N, TY = SH::TY, J = RG + 1, NA = HELM ? 2 : 1;
     constexpr bool ZERO = MODE == kRelax2Zero, UPD = MODE == kRelax2Update;
-    // The z loop is unrolled by three so that the register windows rotate by renaming; with two FP32
-    // cells per thread the three copies (times two groups) outgrow the instruction cache (half of all
+    // The z loop is unrolled by three so that the register windows rotate by renaming; with the cheaper
+    // arithmetic of FP32 levels the three copies (times two groups) outgrow the instruction cache (half of all
     // stalls were instruction fetches), and one copy with about 36 register moves a plane is faster.
-    // Measured (B200, Helmholtz pair): 384^3 326 -> 207 us, ending in the update 394 -> 279; 192^3 48.9 ->
-    // 38.3.
-    constexpr bool kRoll = sizeof(T) == 4 && (PV == 2 || NXT == 192) && !ZERO;
+    // Measured (B200, Helmholtz pair): 384^3 326 -> 207 us, ending in the update 394 -> 279, from zero 221 ->
+    // 161; 192^3 48.9 -> 38.3.
+    constexpr bool kRoll = sizeof(T) == 4;
     static_assert(NXT % 32 == 0, "groups are whole warps");
     static_assert(!(NORM && MODE != kRelax2Plain), "the norm rides on plain passes only");
     static_assert(!UPD || sizeof(T) == 4, "the update pass belongs to mixed precision");
