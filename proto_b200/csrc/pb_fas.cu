@@ -7,11 +7,13 @@
 //   BoxOp_Laplace::flux (DiffCellToFace(d, Lo, 4)) examples/_common/BoxOp_Laplace.H:22-27
 //   averageDown .................................. include/base/implem/Proto_LevelBoxDataImplem.H:993-1038
 // The reference evaluates the operator patch by patch through four temporaries (three face-flux
-// BoxData and a divergence) after an exchange; here every level is one periodic n^3 box without ghost
-// cells (neighbours are read at wrapped offsets: writing two layers of periodic images cost a sweep of a
-// 128^3 level more than its stencil) and one kernel per step evaluates, per cell, the same operations in
-// the same order (face gradients with |=, the divergence with +=, the sum, the flux scale -1), so the
-// residual history and the solution are bitwise the reference's.
+// BoxData and a divergence) after an exchange; here every level is one periodic box and one kernel per
+// step evaluates, per cell, the same operations in the same order (face gradients with |=, the divergence
+// with +=, the sum, the flux scale -1), so the residual history and the solution are bitwise the
+// reference's. A level keeps two ghost columns in x and two ghost rows in y, no ghost planes (the kernels
+// wrap z) and no valid edges or corners between them (no tap reads those): a writer then has at most one
+// image per axis to store beside its cell. With all ghost layers the images cost a sweep of a 128^3 level
+// more than its stencil; with none, resolving every neighbour's wrapped address did.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -27,48 +29,101 @@ PB_DEFINE_ERROR_READER(read_error_fas)
 
 constexpr int kFasGhost = 2;      // reach of the operator
 
-// index of cell (x, y, z) of an n^3 level
+// index of cell (x, y, z) of a plain n^3 field, and of a level's state (x and y may be ghosts)
 __host__ __device__ __forceinline__ long long fas_index(int n, int x, int y, int z)
 {
     return x + (long long)n * (y + (long long)n * z);
+}
+__host__ __device__ __forceinline__ long long fas_state(int n, int x, int y, int z)
+{
+    const int S = n + 2 * kFasGhost;
+    return (x + kFasGhost) + (long long)S * ((y + kFasGhost) + (long long)S * z);
+}
+
+// distance of coordinate c's image on a periodic axis of n >= 4 cells (0: none)
+__device__ __forceinline__ int fas_image(int c, int n) { return c < kFasGhost ? n : (c >= n - kFasGhost ? -n : 0); }
+
+// the ghost cells that are images of the valid cell at q, edges below 4 (several images per axis)
+__device__ __noinline__ void fas_images_small(double* q, int n, int x, int y, double v)
+{
+    const int S = n + 2 * kFasGhost;
+    for (int k = -2; k <= 2; k++) {
+        if (k == 0) continue;
+        if (x + k * n >= -kFasGhost && x + k * n < n + kFasGhost) q[k * n] = v;
+        if (y + k * n >= -kFasGhost && y + k * n < n + kFasGhost) q[k * n * S] = v;
+    }
+}
+
+// v to the valid cell at q and to its ghost images in x and y (SMALL: edges below 4)
+template <bool SMALL>
+__device__ __forceinline__ void fas_store(double* q, int n, int x, int y, double v)
+{
+    *q = v;
+    if constexpr (SMALL) {
+        fas_images_small(q, n, x, y, v);
+        return;
+    }
+    const int ix = fas_image(x, n), iy = fas_image(y, n) * (n + 2 * kFasGhost);
+    if (ix) q[ix] = v;
+    if (iy) q[iy] = v;
 }
 
 // ---- the level passes: epilogues of the march (pb_lap4.cuh); op(u) = -t -------------------------------
 // Jacobi sweep: out = u + (-lambda) * (op(u) + f). FIRST: the level has just
 // been averaged into and f holds only AvgDown(op(u) + f) of the finer level; the coarse force is that
 // minus op of this level's state, which is the op this sweep evaluates anyway, so the sweep completes
-// and stores it (one launch and one pass less per level).
-template <bool FIRST>
+// and stores it (one launch and one pass less per level). Measured (B200, FP64, data in L2): a 128^3 sweep
+// 22.5 -> 17.6 us, 64^3 7.8 -> 5.7.
+// SMALL: edges below 4, where a cell has several images per axis.
+template <bool FIRST, bool SMALL>
 struct EpiFasRelax {
     double* out;
     double* f;
     int n;
     double neg_lambda;
     struct Cursor {
-        long long i;         // (x, y, plane z)
+        double* o;           // (x, y, plane z) of the output state
+        double* f;           // of the force
+        int x, y;
+        int ix, iy0, iy1;    // offsets of the cells' images in x and, row by row, in y (edges >= 4)
         bool a0, a1;
     };
     __device__ __forceinline__ Cursor cursor(int x, int y, int z0, bool a0, bool a1) const
     {
-        return Cursor{fas_index(n, x, y, z0), a0, a1};
+        const int S = n + 2 * kFasGhost;
+        return Cursor{out + fas_state(n, x, y, z0), f + fas_index(n, x, y, z0), x, y,
+                      fas_image(x, n), fas_image(y, n) * S, fas_image(y + 1, n) * S, a0, a1};
     }
     __device__ __forceinline__ void pre(const Cursor& c, int ahead, double& p0, double& p1) const
     {
-        const double* q = f + c.i + (long long)ahead * n * n;
+        const double* q = c.f + (ahead ? n * n : 0);
         if (c.a0) p0 = q[0];
         if (c.a1) p1 = q[n];
     }
     __device__ __forceinline__ void cells(Cursor& c, int, double t0, double t1, double c0, double c1, double p0, double p1) const
     {
+        const int S = n + 2 * kFasGhost;
         if (FIRST) {
             p0 = dadd(p0, t0);
             p1 = dadd(p1, t1);
-            if (c.a0) f[c.i] = p0;
-            if (c.a1) f[c.i + n] = p1;
+            if (c.a0) c.f[0] = p0;
+            if (c.a1) c.f[n] = p1;
         }
-        if (c.a0) out[c.i] = dadd(c0, dmul(neg_lambda, dsub(p0, t0)));
-        if (c.a1) out[c.i + n] = dadd(c1, dmul(neg_lambda, dsub(p1, t1)));
-        c.i += (long long)n * n;
+        const double v0 = dadd(c0, dmul(neg_lambda, dsub(p0, t0))), v1 = dadd(c1, dmul(neg_lambda, dsub(p1, t1)));
+        double* const o1 = c.o + S;
+        if (c.a0) c.o[0] = v0;
+        if (c.a1) o1[0] = v1;
+        if constexpr (SMALL) {
+            if (c.a0) fas_images_small(c.o, n, c.x, c.y, v0);
+            if (c.a1) fas_images_small(o1, n, c.x, c.y + 1, v1);
+        } else {
+            if (c.a0 && c.ix) c.o[c.ix] = v0;
+            if (c.a0 && c.iy0) c.o[c.iy0] = v0;
+            if (c.a1 && c.ix) o1[c.ix] = v1;
+            if (c.a1 && c.iy1) o1[c.iy1] = v1;
+        }
+        c.o += S * S;
+        c.f += n * n;
     }
     __device__ __forceinline__ void end() const {}
 };
@@ -89,7 +144,7 @@ struct EpiFasNorm {
     }
     __device__ __forceinline__ void pre(const Cursor& c, int ahead, double& p0, double& p1) const
     {
-        const double* q = c.f + (long long)ahead * n * n;
+        const double* q = c.f + (ahead ? n * n : 0);
         if (c.a0) p0 = __ldg(q);
         if (c.a1) p1 = __ldg(q + n);
     }
@@ -97,7 +152,7 @@ struct EpiFasNorm {
     {
         if (c.a0) m = upd_abs(m, dsub(p0, t0));
         if (c.a1) m = upd_abs(m, dsub(p1, t1));
-        c.f += (long long)n * n;
+        c.f += n * n;
     }
     __device__ __forceinline__ void end() const { block_max_atomic(m, result); }
 };
@@ -106,6 +161,7 @@ struct EpiFasNorm {
 // c0, and AvgDown(op(u) + f), the first part of the coarse force. A thread's two rows of an even and an
 // odd plane and its x neighbour's (a shuffle away) are a coarse cell's eight children, added in their
 // order; the even lanes keep the sums.
+template <bool SMALL>   // the coarse edge is below 4
 struct EpiFasRestrict {
     const double* f;
     int n;
@@ -124,7 +180,7 @@ struct EpiFasRestrict {
     }
     __device__ __forceinline__ void pre(const Cursor& c, int ahead, double& p0, double& p1) const
     {
-        const double* q = c.f + (long long)ahead * n * n;
+        const double* q = c.f + (ahead ? n * n : 0);
         p0 = __ldg(q);           // idle threads follow a cell of the level, whose edge is even
         p1 = c.y + 1 < n ? __ldg(q + n) : 0.0;
     }
@@ -145,41 +201,74 @@ struct EpiFasRestrict {
             const long long i = fas_index(n / 2, c.x / 2, c.y / 2, z / 2);
             fc[i] = ar;
             c0[i] = au;
-            uc[i] = au;
+            fas_store<SMALL>(uc + fas_state(n / 2, c.x / 2, c.y / 2, z / 2), n / 2, c.x / 2, c.y / 2, au);
         }
-        c.f += (long long)n * n;
+        c.f += n * n;
     }
     __device__ __forceinline__ void end() const {}
 };
 
 // fine correction: u += -(c0 - uc) of the cell's coarse cell (c0: the coarse state as it was averaged,
 // uc: as the coarse cycle left it). A row walk with four planes' loads in flight.
+template <bool SMALL>
 __global__ void __launch_bounds__(kWalkThreads) k_fas_correct(double* u, const double* __restrict__ c0,
                                                               const double* __restrict__ uc, int nf, Walk w)
 {
-    const int nc = nf / 2;
-    const long long nf2 = (long long)nf * nf, nc2 = (long long)nc * nc;
+    const int nc = nf / 2, S = nf + 2 * kFasGhost, Sc = nc + 2 * kFasGhost;
+    const long long nf2 = (long long)S * S, nc2 = (long long)nc * nc, sc2 = (long long)Sc * Sc;
     walk_rows(w, [&](int x, int y, int z, int planes) {          // z is even: planes z, z+1 share a coarse one
-        double* q = u + fas_index(nf, x, y, z);
-        const long long i = fas_index(nc, x / 2, y / 2, z / 2);
+        double* q = u + fas_state(nf, x, y, z);
+        const double* a = c0 + fas_index(nc, x / 2, y / 2, z / 2);
+        const double* b = uc + fas_state(nc, x / 2, y / 2, z / 2);
         double v[kWalkZ], d[kWalkZ / 2];
 #pragma unroll
         for (int k = 0; k < kWalkZ; k++)
             if (k < planes) v[k] = q[k * nf2];
 #pragma unroll
         for (int k = 0; k < kWalkZ / 2; k++)
-            if (2 * k < planes) d[k] = dsub(__ldg(c0 + i + k * nc2), __ldg(uc + i + k * nc2));
+            if (2 * k < planes) d[k] = dsub(__ldg(a + k * nc2), __ldg(b + k * sc2));
 #pragma unroll
         for (int k = 0; k < kWalkZ; k++)
-            if (k < planes) q[k * nf2] = dsub(v[k], d[k / 2]);
+            if (k < planes) fas_store<SMALL>(q + k * nf2, nf, x, y, dsub(v[k], d[k / 2]));
+    });
+}
+
+// n^3 <-> state, x and y ghosts included
+__global__ void __launch_bounds__(kWalkThreads) k_fas_pack(const double* __restrict__ src, double* u, int n, Walk w)
+{
+    const long long S = n + 2 * kFasGhost;
+    walk_rows(w, [&](int x, int y, int z, int planes) {          // x, y of the grown plane
+        const double* q = src + lap4_wrap(x - kFasGhost, n) + (long long)n * (lap4_wrap(y - kFasGhost, n) + (long long)n * z);
+        double* o = u + x + S * (y + S * z);
+        double v[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) v[k] = __ldg(q + (long long)n * n * k);
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) o[S * S * k] = v[k];
+    });
+}
+__global__ void __launch_bounds__(kWalkThreads) k_fas_unpack(const double* __restrict__ u, double* dst, int n, Walk w)
+{
+    const long long S = n + 2 * kFasGhost;
+    walk_rows(w, [&](int x, int y, int z, int planes) {
+        double v[kWalkZ];
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) v[k] = __ldg(u + fas_state(n, x, y, z) + S * S * k);
+#pragma unroll
+        for (int k = 0; k < kWalkZ; k++)
+            if (k < planes) dst[fas_index(n, x, y, z + k)] = v[k];
     });
 }
 
 // ---- the levels of edge <= kFasCoarseEdge in one CTA ------------------------------------------
 // The same per-cell operations as the passes above, in the same order (sweeps, averaging, coarse
 // force, recursion, correction), with every level's state (two buffers), force and averaged copy in
-// shared memory. One launch replaces about thirty launch-bound ones. A 16^3 level keeps its own launches:
-// its sweep is more FP64 work than one SM does in a launch's time (measured with it: 139 us).
+// shared memory, a cell per thread whose neighbours' indices stay in registers. One launch replaces about
+// thirty launch-bound ones: 18 us (46 with the levels in L2 and their images stored). A 16^3 level keeps
+// its own launches: its sweep is more FP64 work than one SM does in a launch's time (with it: 139 us).
 constexpr int kFasCoarseEdge = 8, kFasCoarseMax = 8, kFasCoarseThreads = 512;
 
 struct FasCoarseLevel {
@@ -198,44 +287,53 @@ struct FasCoarseArgs {
 
 #define FAS_BLOCK_LOOP(total) for (int i = threadIdx.x; i < (total); i += blockDim.x)
 
-// body(cell index, t, centre) for every cell of a level, t as in the march
-template <class F>
-__device__ __forceinline__ void fas_blk_cells(const FasCoarseLevel& L, const double* u, F&& body)
-{
-    const int n = L.n;
-    FAS_BLOCK_LOOP(n * n * n)
+// A level has at most one cell per thread (8^3 = 512): the thread's cell and its neighbours' indices
+static_assert(kFasCoarseEdge * kFasCoarseEdge * kFasCoarseEdge <= kFasCoarseThreads, "a thread per cell");
+struct FasCell {
+    int nb[3][4];            // per axis the cells at -2, -1, +1, +2
+    bool in;
+    __device__ __forceinline__ FasCell(int n)
     {
-        const int p[3] = {i % n, i / n % n, i / (n * n)}, step[3] = {1, n, n * n};
-        const double c = u[i];
+        const int i = threadIdx.x, step[3] = {1, n, n * n}, p[3] = {i % n, i / n % n, i / (n * n)};
+        in = i < n * n * n;
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+            for (int o = 0; o < 4; o++)
+                nb[d][o] = in ? i + (lap4_wrap(p[d] + (o < 2 ? o - 2 : o - 1), n) - p[d]) * step[d] : 0;
+    }
+    // t as in the march
+    __device__ __forceinline__ double value(const double* u, double c, const FasCoef& k) const
+    {
         double div = 0.0;
+        const double B = dmul(k.g[1], c);
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            const int base = i - p[d] * step[d];
-            auto at = [&](int o) { return u[base + lap4_wrap(p[d] + o, n) * step[d]]; };
-            const double m2 = at(-2), m1 = at(-1), p1 = at(1), p2 = at(2);
-            const double fp = dsub(dsub(dadd(dmul(L.k.g[0], m1), dmul(L.k.g[1], c)), dmul(L.k.g[1], p1)), dmul(L.k.g[0], p2));
-            const double fm = dsub(dsub(dadd(dmul(L.k.g[0], m2), dmul(L.k.g[1], m1)), dmul(L.k.g[1], c)), dmul(L.k.g[0], p1));
-            div = d == 0 ? dmul(L.k.cp, fp) : dadd(div, dmul(L.k.cp, fp));
-            div = dsub(div, dmul(L.k.cp, fm));
+            const double m2 = u[nb[d][0]], m1 = u[nb[d][1]], p1 = u[nb[d][2]], p2 = u[nb[d][3]];
+            const double Fp = dmul(k.cp, dsub(dsub(dadd(dmul(k.g[0], m1), B), dmul(k.g[1], p1)), dmul(k.g[0], p2)));
+            const double Fm = dmul(k.cp, dsub(dsub(dadd(dmul(k.g[0], m2), dmul(k.g[1], m1)), B), dmul(k.g[0], p1)));
+            div = d == 0 ? Fp : dadd(div, Fp);
+            div = dsub(div, Fm);
         }
-        body(i, dadd(0.0, div), c);
+        return dadd(0.0, div);
     }
-}
+};
 
 // sweeps from buffer `from`; first: the first sweep completes the force (EpiFasRelax)
 __device__ void fas_blk_relax(const FasCoarseLevel& L, double* sm, int from, int sweeps, bool first)
 {
+    const FasCell cell(L.n);
+    const int i = threadIdx.x;
+    const FasCoef k = L.k;
+    double fv = cell.in ? sm[L.f + i] : 0.0;
     int c = from;
-    double* f = sm + L.f;
     for (int s = 0; s < sweeps; s++) {
-        const double* u = sm + L.u[c];
-        double* out = sm + L.u[1 - c];
-        const bool add = first && s == 0;
-        fas_blk_cells(L, u, [&](int i, double t, double centre) {
-            double fv = f[i];
-            if (add) f[i] = fv = dadd(fv, t);
-            out[i] = dadd(centre, dmul(L.neg_lambda, dsub(fv, t)));
-        });
+        if (cell.in) {
+            const double* u = sm + L.u[c];
+            const double centre = u[i], t = cell.value(u, centre, k);
+            if (first && s == 0) sm[L.f + i] = fv = dadd(fv, t);
+            sm[L.u[1 - c] + i] = dadd(centre, dmul(L.neg_lambda, dsub(fv, t)));
+        }
         __syncthreads();
         c = 1 - c;
     }
@@ -249,7 +347,7 @@ __global__ void __launch_bounds__(kFasCoarseThreads) k_fas_coarse_cycle(const __
         const FasCoarseLevel& T = a.lv[a.top];
         FAS_BLOCK_LOOP(T.n * T.n * T.n)
         {
-            sm[T.u[0] + i] = a.u[i];
+            sm[T.u[0] + i] = a.u[fas_state(T.n, i % T.n, i / T.n % T.n, i / (T.n * T.n))];
             sm[T.f + i] = a.f[i];
         }
     }
@@ -266,8 +364,11 @@ __global__ void __launch_bounds__(kFasCoarseThreads) k_fas_coarse_cycle(const __
         const int nf = L.n, nc = C.n;
         const double* u = sm + L.u[c_pre];
         double* res = sm + L.u[1 - c_pre];       // op(u) + f of the fine cells (n^3), until the next sweep
-        const double* f = sm + L.f;
-        fas_blk_cells(L, u, [&](int i, double t, double) { res[i] = dsub(f[i], t); });
+        {
+            const FasCell cell(nf);
+            const int i = threadIdx.x;
+            if (cell.in) res[i] = dsub(sm[L.f + i], cell.value(u, u[i], L.k));
+        }
         __syncthreads();
         FAS_BLOCK_LOOP(nc * nc * nc)
         {
@@ -306,7 +407,7 @@ __global__ void __launch_bounds__(kFasCoarseThreads) k_fas_coarse_cycle(const __
     {
         const FasCoarseLevel& T = a.lv[a.top];
         const double* u = sm + T.u[a.top == 0 ? c_bot : c_end];
-        FAS_BLOCK_LOOP(T.n * T.n * T.n) a.u[i] = u[i];
+        FAS_BLOCK_LOOP(T.n * T.n * T.n) a.u[fas_state(T.n, i % T.n, i / T.n % T.n, i / (T.n * T.n))] = u[i];
     }
 }
 
@@ -315,7 +416,7 @@ struct FasLevel {
     double dx;
     FasCoef k;
     double neg_lambda;
-    double* u[2] = {nullptr, nullptr};   // ping-pong state, n^3
+    double* u[2] = {nullptr, nullptr};   // ping-pong state (fas_state)
     int cur = 0;
     double* f = nullptr;                  // n^3
     double* c0 = nullptr;                 // n^3: copy of the averaged-down state (coarse levels)
@@ -383,7 +484,8 @@ using namespace pb;
 
 static Lap4Geom fas_geom(const FasLevel& L)
 {
-    return Lap4Geom{L.u[L.cur], L.n, (long long)L.n * L.n, L.n, L.n, L.n, 0, 0};
+    const long long S = L.n + 2 * kFasGhost;
+    return Lap4Geom{L.u[L.cur] + fas_state(L.n, 0, 0, 0), S, S * S, L.n, L.n, L.n, 0, 0};
 }
 
 // first: the level's force still lacks its op part (every level below the finest, on the way down)
@@ -393,9 +495,15 @@ static int fas_relax(pb_fas* m, int l, int sweeps, bool first, cudaStream_t st)
     for (int s = 0; s < sweeps; s++) {
         const Lap4Geom g = fas_geom(L);
         double* out = L.u[1 - L.cur];
-        const int e = first && s == 0
-                          ? launch_lap4<true>(g, L.k, EpiFasRelax<true>{out, L.f, L.n, L.neg_lambda}, cached_sm_count(), st)
-                          : launch_lap4<true>(g, L.k, EpiFasRelax<false>{out, L.f, L.n, L.neg_lambda}, cached_sm_count(), st);
+        const int sms = cached_sm_count();
+        const bool fs = first && s == 0;
+        int e;
+        if (L.n < 4)
+            e = fs ? launch_lap4<true>(g, L.k, EpiFasRelax<true, true>{out, L.f, L.n, L.neg_lambda}, sms, st)
+                   : launch_lap4<true>(g, L.k, EpiFasRelax<false, true>{out, L.f, L.n, L.neg_lambda}, sms, st);
+        else
+            e = fs ? launch_lap4<true>(g, L.k, EpiFasRelax<true, false>{out, L.f, L.n, L.neg_lambda}, sms, st)
+                   : launch_lap4<true>(g, L.k, EpiFasRelax<false, false>{out, L.f, L.n, L.neg_lambda}, sms, st);
         if (e != PB_OK) return e;
         L.cur = 1 - L.cur;
     }
@@ -439,11 +547,13 @@ static int fas_vcycle(pb_fas* m, int l, cudaStream_t st)
     int e;
     if ((e = fas_relax(m, l, m->num_pre, !top, st)) != PB_OK) return e;
     C.cur = 0;
-    const EpiFasRestrict r{L.f, L.n, C.u[0], C.c0, C.f, 0.0, 0.0};
-    if ((e = launch_lap4<true>(fas_geom(L), L.k, r, cached_sm_count(), st)) != PB_OK) return e;
+    e = C.n < 4 ? launch_lap4<true>(fas_geom(L), L.k, EpiFasRestrict<true>{L.f, L.n, C.u[0], C.c0, C.f, 0.0, 0.0}, cached_sm_count(), st)
+                : launch_lap4<true>(fas_geom(L), L.k, EpiFasRestrict<false>{L.f, L.n, C.u[0], C.c0, C.f, 0.0, 0.0}, cached_sm_count(), st);
+    if (e != PB_OK) return e;
     if ((e = fas_vcycle(m, l - 1, st)) != PB_OK) return e;
     const Walk w = walk_cube(L.n);
-    k_fas_correct<<<walk_grid(w, 1), kWalkThreads, 0, st>>>(L.u[L.cur], C.c0, C.u[C.cur], L.n, w);
+    if (L.n < 4) k_fas_correct<true><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(L.u[L.cur], C.c0, C.u[C.cur], L.n, w);
+    else k_fas_correct<false><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(L.u[L.cur], C.c0, C.u[C.cur], L.n, w);
     PB_LAUNCH_CHECK();
     return fas_relax(m, l, m->num_post, false, st);
 }
@@ -531,8 +641,10 @@ int pb_fas_create(int n, int num_levels, pb_fas** out)
         // lambda = 0.5 / spectralRadius, spectralRadius = (2*DIM) / dx^2
         L.neg_lambda = -(0.5 / ((2.0 * 3) / std::pow(L.dx, 2)));
         const size_t c = sizeof(double) * (size_t)L.n * L.n * L.n;
-        ok = cudaMalloc(&L.u[0], c) == cudaSuccess && cudaMalloc(&L.u[1], c) == cudaSuccess &&
-             cudaMalloc(&L.f, c) == cudaSuccess && cudaMalloc(&L.c0, c) == cudaSuccess;
+        const size_t g = sizeof(double) * (size_t)(L.n + 2 * kFasGhost) * (L.n + 2 * kFasGhost) * L.n;
+        ok = cudaMalloc(&L.u[0], g) == cudaSuccess && cudaMalloc(&L.u[1], g) == cudaSuccess &&
+             cudaMalloc(&L.f, c) == cudaSuccess && cudaMalloc(&L.c0, c) == cudaSuccess &&
+             cudaMemset(L.u[0], 0, g) == cudaSuccess && cudaMemset(L.u[1], 0, g) == cudaSuccess;
     }
     if (ok) ok = cudaMalloc(&m->d_res, sizeof(double)) == cudaSuccess && cudaMallocHost(&m->h_res, sizeof(double)) == cudaSuccess;
     if (!ok) {
@@ -559,7 +671,10 @@ int pb_fas_solve(pb_fas* m, const double* force, double* phi, int max_iter, doub
     const long long n3 = (long long)T.n * T.n * T.n;
     T.cur = 0;
     PB_CUDA(cudaMemcpyAsync(T.f, force, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
-    PB_CUDA(cudaMemcpyAsync(T.u[0], phi, sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
+    const int S = T.n + 2 * kFasGhost;
+    const Walk wg = walk_of(Region{{0, 0, 0}, {S, S, T.n}}), wv = walk_cube(T.n);
+    k_fas_pack<<<walk_grid(wg, 1), kWalkThreads, 0, st>>>(phi, T.u[0], T.n, wg);
+    PB_LAUNCH_CHECK();
     double r0, r;
     int e;
     if ((e = fas_resnorm(m, st, &r0)) != PB_OK) return e;
@@ -592,7 +707,8 @@ int pb_fas_solve(pb_fas* m, const double* force, double* phi, int max_iter, doub
         if (hist) hist[it] = r;
         if (r < tol * r0) break;
     }
-    PB_CUDA(cudaMemcpyAsync(phi, T.u[T.cur], sizeof(double) * n3, cudaMemcpyDeviceToDevice, st));
+    k_fas_unpack<<<walk_grid(wv, 1), kWalkThreads, 0, st>>>(T.u[T.cur], phi, T.n, wv);
+    PB_LAUNCH_CHECK();
     PB_CUDA(cudaStreamSynchronize(st));
     if (read_error_fas() > 0) return PB_ERR_DEVICE;
     if (iters) *iters = it;

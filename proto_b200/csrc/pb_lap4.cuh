@@ -16,8 +16,9 @@
 // again as they are needed: three operations a cell for 28 registers). With two resident blocks per SM
 // only four warps share a scheduler, so no load may be waited for: a plane's neighbours, and what the
 // epilogue needs, are loaded one plane ahead. All loads are 8 bytes wide from L1-resident rows, so odd
-// sizes and any alignment run the same code. A box reads its ghost cells; a periodic level has none, its
-// threads resolve the wrapped offsets of their x and y neighbours once.
+// sizes and any alignment run the same code. Two cells beyond the range are
+// readable in x and y; in z either too (a box), or the planes wrap (a periodic level, which then needs no
+// images in z).
 #pragma once
 #include <type_traits>
 
@@ -31,8 +32,7 @@ struct FasCoef {
     double cp, c0;   // divergence 1.0*Shift(+e) - 1.0*Shift(0), * 1/dx
 };
 
-// one field as the march sees it: address of cell (0, 0, 0) of the range, pitches, cell counts. A box has
-// two readable cells beyond the range on every side; a periodic level (WRAP) is the range alone.
+// one field as the march sees it: address of cell (0, 0, 0) of the range, pitches, cell counts
 struct Lap4Geom {
     const double* u;
     long long sy, sz;
@@ -91,7 +91,7 @@ __device__ __forceinline__ void lap4_cells(const Lap4Taps& n, const double (&wm)
 // per plane pre(cursor, ahead, p0, p1) loads what it needs of both cells, `ahead` planes above the cursor,
 // cells(cursor, z, t0, t1, c0, c1, p0, p1) takes the rows' t and centre values (every thread of the block
 // calls it, idle ones too) and moves the cursor up; end() once.
-template <bool WRAP, class Epi>
+template <bool WRAPZ, class Epi>
 __global__ void __launch_bounds__(256, 2) k_lap4(const Lap4Geom g, const FasCoef k, Epi epi)
 {
     const int by = blockIdx.x / g.bx;                      // blocks of a plane, x fastest
@@ -101,35 +101,23 @@ __global__ void __launch_bounds__(256, 2) k_lap4(const Lap4Geom g, const FasCoef
     const bool act0 = xr < g.nx && y < g.ny, act1 = xr < g.nx && y + 1 < g.ny;
     // idle threads follow a cell of the range (their loads stay in bounds, nothing is stored)
     const int x = min(xr, g.nx - 1), yc = min(y, g.ny - 1);
-    // offsets of the x neighbours (the same in both rows), of row y+1 and of rows y-2, y-1, y+2, y+3. In a
-    // box, row y+3 may lie past the readable rows when row y+1 is past the range: row y+2 stands in.
-    int xm2 = -2, xm1 = -1, xp1 = 1, xp2 = 2;
-    long long e1 = g.sy, ea = -2 * g.sy, eb = -g.sy, ed = 2 * g.sy, ee = (yc + 3 <= g.ny + 1 ? 3 : 2) * g.sy;
-    if constexpr (WRAP) {
-        xm2 = lap4_wrap(x - 2, g.nx) - x;
-        xm1 = lap4_wrap(x - 1, g.nx) - x;
-        xp1 = lap4_wrap(x + 1, g.nx) - x;
-        xp2 = lap4_wrap(x + 2, g.nx) - x;
-        e1 = (lap4_wrap(yc + 1, g.ny) - yc) * g.sy;
-        ea = (lap4_wrap(yc - 2, g.ny) - yc) * g.sy;
-        eb = (lap4_wrap(yc - 1, g.ny) - yc) * g.sy;
-        ed = (lap4_wrap(yc + 2, g.ny) - yc) * g.sy;
-        ee = (lap4_wrap(yc + 3, g.ny) - yc) * g.sy;
-    }
+    // offsets of rows y+1 and y+3; row y+3 may lie past the readable rows when row y+1 is past the range:
+    // row y+2 stands in
+    const long long e1 = g.sy, ee = (yc + 3 <= g.ny + 1 ? 3 : 2) * g.sy;
     const double* const q0 = g.u + x + g.sy * yc;
-    auto plane = [&](int z) { return q0 + g.sz * (WRAP ? lap4_wrap(z, g.nz) : z); };
+    auto plane = [&](int z) { return q0 + g.sz * (WRAPZ ? lap4_wrap(z, g.nz) : z); };
     auto taps = [&](Lap4Taps& n, const double* q) {
-        n.ya = __ldg(q + ea);
-        n.yb = __ldg(q + eb);
-        n.yd = __ldg(q + ed);
+        n.ya = __ldg(q - 2 * e1);
+        n.yb = __ldg(q - e1);
+        n.yd = __ldg(q + 2 * e1);
         n.ye = __ldg(q + ee);
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             const double* c = q + (r ? e1 : 0);
-            n.xm2[r] = __ldg(c + xm2);
-            n.xm1[r] = __ldg(c + xm1);
-            n.xp1[r] = __ldg(c + xp1);
-            n.xp2[r] = __ldg(c + xp2);
+            n.xm2[r] = __ldg(c - 2);
+            n.xm1[r] = __ldg(c - 1);
+            n.xp1[r] = __ldg(c + 1);
+            n.xp2[r] = __ldg(c + 2);
         }
     };
     typename Epi::Cursor cur = epi.cursor(x, yc, z0, act0, act1);
@@ -153,16 +141,32 @@ __global__ void __launch_bounds__(256, 2) k_lap4(const Lap4Geom g, const FasCoef
             Pz[r] = dmul(k.cp, dsub(dsub(dadd(dmul(k.g[0], m2[r]), dmul(k.g[1], w[0][r])), dmul(k.g[1], w[1][r])),
                                     dmul(k.g[0], w[2][r])));
     }
+    // planes z+1 and z+3, moved up once a step (around the end of a periodic axis)
+    int zn = WRAPZ ? lap4_wrap(z0 + 1, g.nz) : 0, zf = WRAPZ ? lap4_wrap(z0 + 3, g.nz) : 0;
+    const double* qn = q0 + g.sz * (WRAPZ ? zn : z0 + 1);
+    const double* qf = q0 + g.sz * (WRAPZ ? zf : z0 + 3);
+    const long long around = g.sz * g.nz;
     auto step = [&](auto PHc, int z) {
         constexpr int PH = decltype(PHc)::value;
         constexpr int M = PH, C = (PH + 1) & 3, P = (PH + 2) & 3, Q = (PH + 3) & 3, NOW = PH & 1, NEXT = 1 - NOW;
         double far[2] = {0.0, 0.0};
         if (z + 1 < z1) {
-            const double* q3 = plane(z + 3);
 #pragma unroll
-            for (int r = 0; r < 2; r++) far[r] = __ldg(q3 + (r ? e1 : 0));
-            taps(nb[NEXT], plane(z + 1));
+            for (int r = 0; r < 2; r++) far[r] = __ldg(qf + (r ? e1 : 0));
+            taps(nb[NEXT], qn);
             epi.pre(cur, 1, pre[NEXT][0], pre[NEXT][1]);
+            qn += g.sz;
+            qf += g.sz;
+            if constexpr (WRAPZ) {
+                if (++zn == g.nz) {
+                    zn = 0;
+                    qn -= around;
+                }
+                if (++zf == g.nz) {
+                    zf = 0;
+                    qf -= around;
+                }
+            }
         }
         double t[2];
         lap4_cells(nb[NOW], w[M], w[C], w[P], w[Q], Pz, k, t);
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(256, 2) k_lap4(const Lap4Geom g, const FasCoef
 // Launch shape: blocks of 32 x 8 threads (32 x 4 where those leave SMs idle), two resident per SM, and
 // the even z chunk that makes waves x (planes + 3) smallest: a chunk starts with four planes of loads
 // and products beyond its own, worth about three planes.
-template <bool WRAP, class Epi>
+template <bool WRAPZ, class Epi>
 int launch_lap4(Lap4Geom g, const FasCoef& k, const Epi& epi, int sms, cudaStream_t st)
 {
     const long long gx = (g.nx + kLap4Lanes - 1) / kLap4Lanes;
@@ -204,7 +208,7 @@ int launch_lap4(Lap4Geom g, const FasCoef& k, const Epi& epi, int sms, cudaStrea
     }
     while ((g.nz + (long long)g.zd - 1) / g.zd > 65535) g.zd *= 2;
     g.bx = (int)gx;
-    k_lap4<WRAP, Epi><<<dim3((unsigned)plane(), (unsigned)((g.nz + (long long)g.zd - 1) / g.zd)), dim3(kLap4Lanes, rows), 0, st>>>(g, k, epi);
+    k_lap4<WRAPZ, Epi><<<dim3((unsigned)plane(), (unsigned)((g.nz + (long long)g.zd - 1) / g.zd)), dim3(kLap4Lanes, rows), 0, st>>>(g, k, epi);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
