@@ -139,10 +139,12 @@ __global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ sr
 // planes, and only the previous, the current and the next plane (on its way, a whole step early) are in
 // registers. Bound by FP64 issue (27 multiplies and 27 adds, each rounded: 12 us at 3.95 M cells) and
 // load latency. Measured (B200, two components of 193 x 161 x 127 FP64 cells): 68 us a component one cell
-// per thread, 43 with the three planes held, 33 with the next plane loaded a step early. Below kCubeMin cells the columns are too few to fill the GPU, and the table kernel takes
+// per thread, 43 with the three planes held, 33 with the next plane loaded a step early, 28 with four more
+// asked into L2. Below kCubeMin cells the columns are too few to fill the GPU, and the table kernel takes
 // four cells per thread.
 constexpr long long kCubeMin = 1 << 17;
 constexpr int kCubeThreads = 128, kCubePerSm = 5;
+constexpr int kCubePrefetch = 4;   // planes past the next one whose lines are asked into L2
 template <typename T>
 struct CubeArgs {
     T c[27];                    // by cube position (z+1)*9 + (y+1)*3 + (x+1)
@@ -173,7 +175,8 @@ __global__ void __launch_bounds__(kCubeThreads, kCubePerSm) k_cube(FieldView<con
         // plane z of the chunk in cur, z - 1 in prev, z + 1 on its way into next: completes cell z - 1
         // (its upper plane), then starts cell z
         auto step = [&](const T* prev, const T* cur, T* next, int z) {
-            if (z < z1) load(next);
+            if (z < z1) load(next);               // moves q to plane z + 2
+            if (z + 1 + kCubePrefetch <= z1) prefetch_l2(q + (kCubePrefetch - 1) * s.sz);
             if (z > z0) {
 #pragma unroll
                 for (int k = 18; k < 27; k++) term(acc, k, cur[k - 18]);
@@ -190,6 +193,9 @@ __global__ void __launch_bounds__(kCubeThreads, kCubePerSm) k_cube(FieldView<con
             }
         };
         T p0[9], p1[9], p2[9];
+#pragma unroll
+        for (int k = 0; k <= kCubePrefetch; k++)
+            if (z0 + k <= z1) prefetch_l2(q + (k + 1) * s.sz);
         load(p0);
         load(p1);
         for (int z = z0; z <= z1; z += 3) {
