@@ -74,13 +74,17 @@ __device__ __forceinline__ void fas_store(double* q, int n, int x, int y, double
 // minus op of this level's state, which is the op this sweep evaluates anyway, so the sweep completes
 // and stores it (one launch and one pass less per level). Measured (B200, FP64, data in L2): a 128^3 sweep
 // 22.5 -> 17.6 us, 64^3 7.8 -> 5.7.
-// SMALL: edges below 4, where a cell has several images per axis.
-template <bool FIRST, bool SMALL>
+// SMALL: edges below 4, where a cell has several images per axis. NORM: also max |op(u) + f| of the state
+// the sweep starts from, into result (Reduction<Abs>: NaN ignored): the solver's test of a cycle rides on
+// the next cycle's first sweep, which writes the other buffer, so the state measured stays intact.
+template <bool FIRST, bool SMALL, bool NORM = false>
 struct EpiFasRelax {
     double* out;
     double* f;
     int n;
     double neg_lambda;
+    double* result = nullptr;
+    double m = 0.0;
     struct Cursor {
         double* o;           // (x, y, plane z) of the output state
         double* f;           // of the force
@@ -100,9 +104,13 @@ struct EpiFasRelax {
         if (c.a0) p0 = q[0];
         if (c.a1) p1 = q[n];
     }
-    __device__ __forceinline__ void cells(Cursor& c, int, double t0, double t1, double c0, double c1, double p0, double p1) const
+    __device__ __forceinline__ void cells(Cursor& c, int, double t0, double t1, double c0, double c1, double p0, double p1)
     {
         const int S = n + 2 * kFasGhost;
+        if (NORM) {
+            if (c.a0) m = upd_abs(m, dsub(p0, t0));
+            if (c.a1) m = upd_abs(m, dsub(p1, t1));
+        }
         if (FIRST) {
             p0 = dadd(p0, t0);
             p1 = dadd(p1, t1);
@@ -125,36 +133,10 @@ struct EpiFasRelax {
         c.o += S * S;
         c.f += n * n;
     }
-    __device__ __forceinline__ void end() const {}
-};
-
-// max |op(u) + f|  (Reduction<Abs>: NaN ignored)
-struct EpiFasNorm {
-    const double* f;
-    int n;
-    double* result;
-    double m;
-    struct Cursor {
-        const double* f;
-        bool a0, a1;
-    };
-    __device__ __forceinline__ Cursor cursor(int x, int y, int z0, bool a0, bool a1) const
+    __device__ __forceinline__ void end() const
     {
-        return Cursor{f + x + (long long)n * (y + (long long)n * z0), a0, a1};
+        if (NORM) block_max_atomic(m, result);
     }
-    __device__ __forceinline__ void pre(const Cursor& c, int ahead, double& p0, double& p1) const
-    {
-        const double* q = c.f + (ahead ? n * n : 0);
-        if (c.a0) p0 = __ldg(q);
-        if (c.a1) p1 = __ldg(q + n);
-    }
-    __device__ __forceinline__ void cells(Cursor& c, int, double t0, double t1, double, double, double p0, double p1)
-    {
-        if (c.a0) m = upd_abs(m, dsub(p0, t0));
-        if (c.a1) m = upd_abs(m, dsub(p1, t1));
-        c.f += n * n;
-    }
-    __device__ __forceinline__ void end() const { block_max_atomic(m, result); }
 };
 
 // To the coarser level, in one pass over the finer: coarse state = AvgDown(u) and its copy
@@ -537,15 +519,17 @@ static int fas_coarse(pb_fas* m, int l, cudaStream_t st)
     return PB_OK;
 }
 
+// The finest level's first sweep has been done by the norm pass that measured its state.
 static int fas_vcycle(pb_fas* m, int l, cudaStream_t st)
 {
     const bool top = l == (int)m->lv.size() - 1;
+    const int done = top ? 1 : 0;
     if (m->lv[l].n <= kFasCoarseEdge && l < kFasCoarseMax && !top) return fas_coarse(m, l, st);
-    if (l == 0) return fas_relax(m, l, m->num_bottom, !top, st);
+    if (l == 0) return fas_relax(m, l, m->num_bottom - done, !top, st);
     FasLevel& L = m->lv[l];
     FasLevel& C = m->lv[l - 1];
     int e;
-    if ((e = fas_relax(m, l, m->num_pre, !top, st)) != PB_OK) return e;
+    if ((e = fas_relax(m, l, m->num_pre - done, !top, st)) != PB_OK) return e;
     C.cur = 0;
     e = C.n < 4 ? launch_lap4<true>(fas_geom(L), L.k, EpiFasRestrict<true>{L.f, L.n, C.u[0], C.c0, C.f, 0.0, 0.0}, cached_sm_count(), st)
                 : launch_lap4<true>(fas_geom(L), L.k, EpiFasRestrict<false>{L.f, L.n, C.u[0], C.c0, C.f, 0.0, 0.0}, cached_sm_count(), st);
@@ -558,12 +542,16 @@ static int fas_vcycle(pb_fas* m, int l, cudaStream_t st)
     return fas_relax(m, l, m->num_post, false, st);
 }
 
-// max |op(u) + f| on the finest level into the pinned host word (stream ordered, no wait)
+// max |op(u) + f| on the finest level into the pinned host word (stream ordered, no wait), fused with the
+// next cycle's first sweep into the other buffer; T.cur stays on the state measured
 static int fas_enqueue_resnorm(pb_fas* m, cudaStream_t st)
 {
     FasLevel& T = m->lv.back();
     PB_CUDA(cudaMemsetAsync(m->d_res, 0, sizeof(double), st));
-    const int e = launch_lap4<true>(fas_geom(T), T.k, EpiFasNorm{T.f, T.n, m->d_res, 0.0}, cached_sm_count(), st);
+    double* out = T.u[1 - T.cur];
+    const int sms = cached_sm_count();
+    const int e = T.n < 4 ? launch_lap4<true>(fas_geom(T), T.k, EpiFasRelax<false, true, true>{out, T.f, T.n, T.neg_lambda, m->d_res}, sms, st)
+                          : launch_lap4<true>(fas_geom(T), T.k, EpiFasRelax<false, false, true>{out, T.f, T.n, T.neg_lambda, m->d_res}, sms, st);
     if (e != PB_OK) return e;
     PB_CUDA(cudaMemcpyAsync(m->h_res, m->d_res, sizeof(double), cudaMemcpyDeviceToHost, st));
     return PB_OK;
@@ -580,6 +568,7 @@ static int fas_resnorm(pb_fas* m, cudaStream_t st, double* out)
 
 static int fas_cycle_and_norm(pb_fas* m, cudaStream_t st)
 {
+    m->lv.back().cur = 1 - m->lv.back().cur;   // on from the sweep that the last norm pass did
     const int e = fas_vcycle(m, (int)m->lv.size() - 1, st);
     return e != PB_OK ? e : fas_enqueue_resnorm(m, st);
 }
