@@ -414,7 +414,6 @@ static FasCoef fas_coefs(double dx)
         k.g[t] = (s != 1.0) ? c * s : c;
     }
     k.cp = (s != 1.0) ? 1.0 * s : 1.0;
-    k.c0 = (s != 1.0) ? -1.0 * s : -1.0;
     return k;
 }
 

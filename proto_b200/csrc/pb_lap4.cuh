@@ -29,7 +29,7 @@ namespace pb {
 
 struct FasCoef {
     double g[4];     // DiffCellToFace(d, Lo, 4) * 1/dx, offsets -2, -1, 0, +1 along d
-    double cp, c0;   // divergence 1.0*Shift(+e) - 1.0*Shift(0), * 1/dx
+    double cp;       // divergence 1.0*Shift(+e) - 1.0*Shift(0), * 1/dx: +cp and -cp
 };
 
 // one field as the march sees it: address of cell (0, 0, 0) of the range, pitches, cell counts
