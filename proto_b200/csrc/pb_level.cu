@@ -466,6 +466,15 @@ __global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const 
 #pragma unroll
             for (int r = 0; r < 2; r++) w[r][k] = zcol(z0 - R + k, r);
     }
+    // The last row of a patch of odd y extent has no second row: row y + 1, its +y tap, is the next patch's
+    // first. From plane z0 + R on the ring holds it; the planes before come from that patch here.
+    if (act && !act1) {
+        const long long Sq = t.nb_S[1][1];
+        const double* q = u + t.nb_off[1][1] + (x + g0) + Sx * (g1 + Sq * (z0 + g2));
+#pragma unroll
+        for (int k = 0; k < R; k++)
+            if (z0 + k < z1) w[1][R + k] = __ldg(reinterpret_cast<const double2*>(q + Sx * Sq * k));
+    }
     double* op = out + t.off + cxy + Sxy * t.z0;
     const int sc = (2 * ly + R) * BX + (2 * lx + R);   // even: pairs are 16-byte aligned in the ring
     auto ring2 = [&](const double* q) { return *reinterpret_cast<const double2*>(q); };

@@ -205,3 +205,29 @@ def test_fused_steps_other_kernels_equal_the_exchange_loop(golden, pb, case):
     torch.cuda.synchronize()
     pb.device_check()
     assert np.array_equal(_valid(lv, a.cpu().numpy()), _valid(lv, a2.cpu().numpy()))
+
+
+@pytest.mark.parametrize("tune", [False, True])
+@pytest.mark.parametrize("epilogue", [0, 2])
+def test_pair_steps_at_odd_y_extents(golden, pb, epilogue, tune):
+    """Even x and odd y extents: the two-row kernel's last row of a patch has no partner, and its +y
+    neighbours lie in the next patch. Odd z extents leave chunks of one and a few planes. Bitwise the
+    exchange + stencil loop (epilogue 0: the plain application)."""
+    import torch
+    widths = [[16, 24, 64], [15, 17, 3, 8], [16, 33, 3, 17]]
+    lv, S, _, u, a, L = _level13(golden, pb, widths, 17)
+    b = torch.zeros_like(a)
+    h = 1.0 / L[0]
+    scale, dt = (1.0 / (h * h), 0.1 * h * h) if epilogue else (0.25, 0.0)
+    if tune:
+        lv.autotune(S, a.clone(), b, scale=scale)
+    a2, b2 = a.clone(), b.clone()
+    lv.steps(S, epilogue, a, b, 3, scale=scale, a=dt)
+    for _ in range(3):
+        lv.exchange(a2)
+        lv.stencil(S, epilogue, a2, b2, scale=scale, a=dt)
+        a2, b2 = b2, a2
+    torch.cuda.synchronize()
+    pb.device_check()
+    # an odd number of steps: the result is in the first slab either way
+    assert np.array_equal(_valid(lv, a.cpu().numpy()), _valid(lv, a2.cpu().numpy()))
