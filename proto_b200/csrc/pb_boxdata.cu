@@ -11,6 +11,8 @@
 // with several planes' loads in flight.
 #include <cfloat>
 #include <cstring>
+#include <mutex>
+#include <new>
 
 #include "pb_internal.cuh"
 #include "pb_stencil_impl.cuh"
@@ -227,29 +229,218 @@ __global__ void __launch_bounds__(kWalkThreads) k_interp_const(int ratio, const 
     });
 }
 
-// ---- reduction scratch (per process, per device 0..15) ----------------------------------------
-struct RedScratch {
-    double* partials = nullptr;
+// ---- reduction scratch ------------------------------------------------------------------------
+// A slot is what one reduction needs while it is in flight: partial results, a ticket and, for calls
+// that wait, a page-locked result word (written by the kernel: no copy to fetch it). Calls come from
+// several threads and on several streams, so no two reductions in flight share a slot:
+//   * a call that waits takes an idle slot and gives it back after its synchronise;
+//   * an asynchronous call uses its stream's slot, and its kernel waits (on the device) for the event that
+//     the slot's last kernel recorded: nothing to wait for on the same stream, and right when a stream's
+//     handle comes back or streams beyond kRedStreams take over a slot;
+//   * a captured call's slot belongs to the graph, which may run at any time beside other reductions,
+//     and becomes idle when the graph and its executables are gone.
+struct RedSlot {
+    double* partials = nullptr;    // kRedBlocks
     unsigned int* ticket = nullptr;
-    double* result = nullptr;      // page-locked host memory that the kernel writes (no copy to fetch it)
+    double* result = nullptr;      // allocated when a call that waits first takes the slot
+    cudaEvent_t done = nullptr;    // after the last kernel (slots of streams)
+    RedSlot* next = nullptr;       // idle list
+    int device = 0;
 };
-static RedScratch g_red[16];
-
-static int red_scratch(RedScratch** out)
+constexpr int kRedDevices = 16, kRedStreams = 32, kRedIdleMax = 64;
+struct RedPool {
+    std::mutex mutex;
+    RedSlot* idle = nullptr;
+    int nidle = 0;
+    cudaStream_t stream[kRedStreams];
+    RedSlot* of_stream[kRedStreams] = {};
+    unsigned evict = 0;
+};
+// not destroyed: a graph may give its slot back while the process exits
+static RedPool* red_pools()
 {
-    int dev = 0;
-    PB_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16) return PB_ERR_UNSUPPORTED;
-    RedScratch& s = g_red[dev];
-    if (!s.partials) {
-        if (!s.result) PB_CUDA(cudaHostAlloc(&s.result, sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
-        if (!s.ticket) {
-            PB_CUDA(cudaMalloc(&s.ticket, sizeof(unsigned int)));
-            PB_CUDA(cudaMemset(s.ticket, 0, sizeof(unsigned int)));
-        }
-        PB_CUDA(cudaMalloc(&s.partials, kRedBlocks * sizeof(double)));   // last: its address says the scratch is whole
+    static RedPool* p = new (std::nothrow) RedPool[kRedDevices];
+    return p;
+}
+
+// Allocating and freeing are forbidden while this thread (or, in the global mode, any thread) captures,
+// unless the thread says that it is not part of the capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static void red_free(RedSlot* s)
+{
+    if (!s) return;
+    RelaxedCapture relaxed;
+    cudaFree(s->partials);
+    if (s->result) cudaFreeHost(s->result);
+    if (s->done) cudaEventDestroy(s->done);
+    delete s;
+}
+
+static cudaError_t red_alloc(RedSlot* s)
+{
+    RelaxedCapture relaxed;
+    cudaStream_t st;
+    const size_t bytes = kRedBlocks * sizeof(double) + 256;
+    cudaError_t e = cudaMalloc(&s->partials, bytes);
+    if (e != cudaSuccess) return e;
+    s->ticket = reinterpret_cast<unsigned int*>(s->partials + kRedBlocks);
+    // cleared on a stream of its own: the caller's may be capturing
+    if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) return e;
+    e = cudaMemsetAsync(s->partials, 0, bytes, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaStreamDestroy(st);
+    return e;
+}
+
+static int red_new(int dev, RedSlot** out)
+{
+    RedSlot* s = new (std::nothrow) RedSlot;
+    if (!s) return PB_ERR_NOMEM;
+    s->device = dev;
+    const cudaError_t e = red_alloc(s);
+    if (e != cudaSuccess) {
+        red_free(s);
+        set_cuda_error(e);
+        return PB_ERR_CUDA;
     }
-    *out = &s;
+    *out = s;
+    return PB_OK;
+}
+
+static int red_pool(int* dev, RedPool** out)
+{
+    PB_CUDA(cudaGetDevice(dev));
+    if (*dev < 0 || *dev >= kRedDevices) return PB_ERR_UNSUPPORTED;
+    RedPool* p = red_pools();
+    if (!p) return PB_ERR_NOMEM;
+    *out = p + *dev;
+    return PB_OK;
+}
+
+// an idle slot of the current device, or a new one
+static int red_take(RedSlot** out)
+{
+    int dev;
+    RedPool* p;
+    const int e = red_pool(&dev, &p);
+    if (e != PB_OK) return e;
+    {
+        std::lock_guard<std::mutex> lock(p->mutex);
+        if (p->idle) {
+            *out = p->idle;
+            p->idle = p->idle->next;
+            p->nidle--;
+            return PB_OK;
+        }
+    }
+    return red_new(dev, out);
+}
+
+static void red_idle(RedSlot* s)
+{
+    RedPool* p = red_pools() + s->device;
+    std::lock_guard<std::mutex> lock(p->mutex);
+    s->next = p->idle;
+    p->idle = s;
+    p->nidle++;
+}
+
+// back from a call that waited; idle slots above the limit are freed here (a graph's destructor may not)
+static void red_give(RedSlot* s)
+{
+    red_idle(s);
+    RedPool* p = red_pools() + s->device;
+    RedSlot* extra = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(p->mutex);
+        if (p->nidle > kRedIdleMax) {
+            extra = p->idle;
+            p->idle = extra->next;
+            p->nidle--;
+        }
+    }
+    red_free(extra);
+}
+static void CUDART_CB red_graph_gone(void* s) { red_idle(static_cast<RedSlot*>(s)); }
+
+// The fold itself, with the scratch of slot s.
+static int launch_reduce(int op, const double* data, const Box3& b, const Box3& r, RedSlot* s, double* result, cudaStream_t st)
+{
+    Region rg;                           // an empty intersection folds nothing: the operation's initial value
+    if (bempty(r)) { rg.lo[0] = b.lo[0]; rg.lo[1] = b.lo[1]; rg.lo[2] = b.lo[2]; rg.n[0] = rg.n[1] = rg.n[2] = 0; }
+    else rg = region_of(r);
+    const Walk w = walk_of(rg);
+    const int rows = kRedThreads >> w.lx;
+    const long long tiles = (long long)((w.ny + rows - 1) / rows) * ((w.nz + kRedZ - 1) / kRedZ);
+    int grid = tiles < kRedBlocks ? (int)tiles : kRedBlocks;
+    if (grid < 1) grid = 1;
+    const FieldView<const double> f = view_of(data, b, rg);
+    switch (op) {
+        case 0: k_reduce<0><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        case 1: k_reduce<1><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        case 2: k_reduce<2><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        case 3: k_reduce<3><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        case 4: k_reduce<4><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        default: k_reduce<5><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+    }
+    PB_LAUNCH_CHECK();
+    return PB_OK;
+}
+
+// on the capturing stream: the graph keeps the slot
+static int reduce_captured(int op, const double* data, const Box3& b, const Box3& r, double* result, cudaGraph_t graph,
+                           cudaStream_t st)
+{
+    RedSlot* s;
+    int e = red_take(&s);
+    if (e != PB_OK) return e;
+    cudaUserObject_t keep;
+    cudaError_t ce = cudaUserObjectCreate(&keep, s, red_graph_gone, 1, cudaUserObjectNoDestructorSync);
+    if (ce != cudaSuccess) {
+        red_idle(s);
+        set_cuda_error(ce);
+        return PB_ERR_CUDA;
+    }
+    ce = cudaGraphRetainUserObject(graph, keep, 1, cudaGraphUserObjectMove);
+    if (ce != cudaSuccess) {
+        cudaUserObjectRelease(keep, 1);      // gives the slot back
+        set_cuda_error(ce);
+        return PB_ERR_CUDA;
+    }
+    return launch_reduce(op, data, b, r, s, result, st);
+}
+
+static int reduce_on_stream(int op, const double* data, const Box3& b, const Box3& r, double* result, cudaStream_t st)
+{
+    int dev;
+    RedPool* p;
+    int e = red_pool(&dev, &p);
+    if (e != PB_OK) return e;
+    std::lock_guard<std::mutex> lock(p->mutex);
+    int k = 0;
+    while (k < kRedStreams && p->of_stream[k] && p->stream[k] != st) k++;
+    if (k == kRedStreams) k = p->evict++ % kRedStreams;
+    RedSlot*& s = p->of_stream[k];
+    p->stream[k] = st;
+    if (!s) {
+        RedSlot* fresh;
+        if ((e = red_new(dev, &fresh)) != PB_OK) return e;
+        const cudaError_t ce = cudaEventCreateWithFlags(&fresh->done, cudaEventDisableTiming);
+        if (ce != cudaSuccess) {
+            red_free(fresh);
+            set_cuda_error(ce);
+            return PB_ERR_CUDA;
+        }
+        s = fresh;
+    }
+    PB_CUDA(cudaStreamWaitEvent(st, s->done, 0));
+    if ((e = launch_reduce(op, data, b, r, s, result, st)) != PB_OK) return e;
+    PB_CUDA(cudaEventRecord(s->done, st));
     return PB_OK;
 }
 
@@ -345,42 +536,44 @@ int pb_reduce_async_f64(int op, const double* data, pb_box box, pb_box region, d
     Box3 b = to_box(box), r = to_box(region);
     if (bempty(b)) return PB_ERR_BOX;
     r = bempty(r) ? b : intersect(r, b);
-    RedScratch* s;
-    int e = red_scratch(&s);
-    if (e != PB_OK) return e;
-    Region rg;                           // an empty intersection folds nothing: the operation's initial value
-    if (bempty(r)) { rg.lo[0] = b.lo[0]; rg.lo[1] = b.lo[1]; rg.lo[2] = b.lo[2]; rg.n[0] = rg.n[1] = rg.n[2] = 0; }
-    else rg = region_of(r);
-    const Walk w = walk_of(rg);
-    const int rows = kRedThreads >> w.lx;
-    const long long tiles = (long long)((w.ny + rows - 1) / rows) * ((w.nz + kRedZ - 1) / kRedZ);
-    int grid = tiles < kRedBlocks ? (int)tiles : kRedBlocks;
-    if (grid < 1) grid = 1;
-    const FieldView<const double> f = view_of(data, b, rg);
     cudaStream_t st = (cudaStream_t)stream;
-    switch (op) {
-        case 0: k_reduce<0><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-        case 1: k_reduce<1><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-        case 2: k_reduce<2><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-        case 3: k_reduce<3><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-        case 4: k_reduce<4><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-        default: k_reduce<5><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result_dev); break;
-    }
-    PB_LAUNCH_CHECK();
-    return PB_OK;
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t graph = nullptr;
+    PB_CUDA(cudaStreamGetCaptureInfo_v2(st, &cs, nullptr, &graph, nullptr, nullptr));
+    return cs == cudaStreamCaptureStatusActive ? reduce_captured(op, data, b, r, result_dev, graph, st)
+                                               : reduce_on_stream(op, data, b, r, result_dev, st);
 }
 
 int pb_reduce_f64(int op, const double* data, pb_box box, pb_box region, double* result, void* stream)
 {
-    if (!result) return PB_ERR_ARG;
-    RedScratch* s;
-    int e = red_scratch(&s);
+    if (!data || !result || op < 0 || op > 5) return PB_ERR_ARG;
+    Box3 b = to_box(box), r = to_box(region);
+    if (bempty(b)) return PB_ERR_BOX;
+    r = bempty(r) ? b : intersect(r, b);
+    RedSlot* s;
+    int e = red_take(&s);
     if (e != PB_OK) return e;
-    e = pb_reduce_async_f64(op, data, box, region, s->result, stream);
-    if (e != PB_OK) return e;
-    PB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    *result = *(volatile double*)s->result;
-    return PB_OK;
+    if (!s->result) {
+        RelaxedCapture relaxed;
+        const cudaError_t ce = cudaHostAlloc(&s->result, sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable);
+        if (ce != cudaSuccess) {
+            s->result = nullptr;
+            red_idle(s);
+            set_cuda_error(ce);
+            return PB_ERR_CUDA;
+        }
+    }
+    e = launch_reduce(op, data, b, r, s, s->result, (cudaStream_t)stream);
+    if (e == PB_OK) {
+        const cudaError_t ce = cudaStreamSynchronize((cudaStream_t)stream);
+        if (ce != cudaSuccess) {       // the kernel may still run (or was captured): the slot is not given back
+            set_cuda_error(ce);
+            return PB_ERR_CUDA;
+        }
+        *result = *(volatile double*)s->result;
+    }
+    red_give(s);
+    return e;
 }
 
 int pb_interp_constant_f64(int ratio, const double* src, pb_box src_box, double* dst, pb_box dst_box, int overwrite,
