@@ -125,7 +125,7 @@ int pb_forall_axpby_f64(double* out, pb_box out_box, const double* x, pb_box x_b
  * pb_reduce_f64 waits for the result (Reduction::fetch); the _async form leaves the result in
  * device memory. Max/Min/Abs are exact; sums use a fixed two-level tree (deterministic run to run).
  * Both may be called from several threads and on several streams at once: each call in flight has
- * scratch of its own (8 KB, kept for later calls). A captured pb_reduce_async_f64 takes scratch that
+ * scratch of its own (3 KB, kept for later calls). A captured pb_reduce_async_f64 takes scratch that
  * lives as long as the graph. */
 int pb_reduce_f64(int op, const double* data, pb_box box, pb_box region, double* result, void* stream);
 int pb_reduce_async_f64(int op, const double* data, pb_box box, pb_box region, double* result_dev,

@@ -13,6 +13,8 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
+#include <utility>
 
 #include "pb_internal.cuh"
 #include "pb_stencil_impl.cuh"
@@ -38,7 +40,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_binop(FieldView<double> d, lon
     for (int c = blockIdx.z; c < ncomp; c += gridDim.z) {
         double* dp = d.p + c * dvol;
         const double* sp = s.p + c * svol;
-        walk_rows(w, [&](int x, int y, int z, int planes) {
+        walk_items(w, [&](int x, int y, int z, int planes) {
             double* dq = dp + x + d.sy * y + d.sz * z;
             const double* sq = sp + x + s.sy * y + s.sz * z;
             double sv[kWalkZ], dv[kWalkZ];
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_scalar(FieldView<double> d, lo
 {
     for (int c = blockIdx.z; c < ncomp; c += gridDim.z) {
         double* dp = d.p + c * dvol;
-        walk_rows(w, [&](int x, int y, int z, int planes) {
+        walk_items(w, [&](int x, int y, int z, int planes) {
             double* dq = dp + x + d.sy * y + d.sz * z;
             double dv[kWalkZ];
 #pragma unroll
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_scalar(FieldView<double> d, lo
 __global__ void __launch_bounds__(kWalkThreads) k_axpby(FieldView<double> o, FieldView<const double> xs,
                                                         FieldView<const double> ys, Walk w, double a, double b)
 {
-    walk_rows(w, [&](int x, int y, int z, int planes) {
+    walk_items(w, [&](int x, int y, int z, int planes) {
         double* oq = o.p + x + o.sy * y + o.sz * z;
         const double* xq = xs.p + x + xs.sy * y + xs.sz * z;
         const double* yq = ys.p + x + ys.sy * y + ys.sz * z;
@@ -96,11 +98,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_axpby(FieldView<double> o, Fie
 
 // ---- reductions ---------------------------------------------------------------------------------
 // Pass 1: every block folds its share; pass 2 (the last block to finish, found through an atomic
-// ticket) folds the per-block partials in block order, so sums are deterministic. A share is a fixed
-// set of tiles (a block's rows x kRedZ planes), walked like the pointwise kernels: each thread keeps kRedZ
-// loads in flight, one accumulator per plane of the tile. (Sharing a row between blocks, as those kernels
-// do, was slower: 11.0 -> 13.5 us at 160^3; the last block has more partial results to fold.)
-constexpr int kRedBlocks = 1024;
+// ticket) folds the per-block partials in block order, so sums are deterministic. A share is a run of
+// consecutive items of kRedZ planes (pb_walk.cuh): a thread has the loads of two items in flight and one
+// accumulator per plane. Two blocks per SM: more partial results cost the last block more than the extra
+// warps give (160^3: 592 blocks 8.5 us, 296 7.8). The number is fixed, so a result does not depend on the GPU.
+// Boxes thin in z fold along y, and lines take kRedZ single cells a thread. Measured (B200, us): square
+// sum of 160^3 7.9, 256^3 33; maximum norm of a line of 2^20 cells 6.2, of 2048 x 2048 x 1 8.2, each the
+// same along any axis.
+constexpr int kRedBlocks = 296;
 constexpr int kRedThreads = 256;
 constexpr int kRedZ = 8;
 
@@ -115,7 +120,7 @@ __device__ __forceinline__ double red_upd(int op, double v1, double v2)
         case 1: return (v2 < v1) ? v2 : v1;                 // std::min
         case 2: return upd_abs(v1, v2);
         case 3: return dadd(v1, v2);
-        case 4: return dadd(v1, v2 > 0 ? v2 : -v2);
+        case 4: return dadd(v1, fabs(v2));
         default: return dadd(v1, dmul(v2, v2));
     }
 }
@@ -144,33 +149,53 @@ __device__ double block_reduce(int op, double v)
     return v;
 }
 
-// OP is a template argument so that the fold is one instruction or two, not a switch per cell.
-template <int op>
-__global__ void __launch_bounds__(kRedThreads) k_reduce(FieldView<const double> f, Walk w, double* partials,
+// OP is a template argument so that the fold is one instruction or two, not a switch per cell. chunk: items
+// of a block. LINE: items are single cells.
+template <int op, bool LINE>
+__global__ void __launch_bounds__(kRedThreads) k_reduce(FieldView<const double> f, Walk w, long long chunk, double* partials,
                                                         unsigned int* ticket, double* result)
 {
     double acc[kRedZ];
 #pragma unroll
     for (int k = 0; k < kRedZ; k++) acc[k] = red_init(op);
-    const int rows = kRedThreads >> w.lx;
-    const int lane = threadIdx.x & ((1 << w.lx) - 1), row = threadIdx.x >> w.lx;
-    const int ty = (w.ny + rows - 1) / rows, tz = (w.nz + kRedZ - 1) / kRedZ;
-    const long long tiles = (long long)ty * tz;
-    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int y = (int)(t % ty) * rows + row, z = (int)(t / ty) * kRedZ;
-        if (y >= w.ny) continue;
-        const double* q = f.p + f.sy * y + f.sz * z;
-        const int planes = min(kRedZ, w.nz - z);
-        for (int x = lane; x < w.nx; x += 1 << w.lx) {
-            double v[kRedZ];
+    auto fold = [&](auto first, auto step, auto end) {       // 32- or 64-bit item numbers
+        if constexpr (LINE) {
+            for (auto i = first; i < end; i += kRedZ * step) {
+                double v[kRedZ];
 #pragma unroll
-            for (int k = 0; k < kRedZ; k++)
-                if (k < planes) v[k] = __ldg(q + x + k * f.sz);
+                for (int k = 0; k < kRedZ; k++) {
+                    const auto j = i + k * step;
+                    int x, y, z;
+                    if (j < end) {
+                        walk_item(w, j, x, y, z);
+                        v[k] = __ldg(f.p + x + f.sy * y + f.sz * z);
+                    }
+                }
 #pragma unroll
-            for (int k = 0; k < kRedZ; k++)
-                if (k < planes) acc[k] = red_upd(op, acc[k], v[k]);
+                for (int k = 0; k < kRedZ; k++)
+                    if (i + k * step < end) acc[k] = red_upd(op, acc[k], v[k]);
+            }
+        } else {
+#pragma unroll 2
+            for (auto i = first; i < end; i += step) {
+                int x, y, g;
+                walk_item(w, i, x, y, g);
+                const double* q = f.p + x + f.sy * y + f.sz * (g * kRedZ);
+                const int planes = min(kRedZ, w.nz - g * kRedZ);
+                double v[kRedZ];
+#pragma unroll
+                for (int k = 0; k < kRedZ; k++)
+                    if (k < planes) v[k] = __ldg(q + k * f.sz);
+#pragma unroll
+                for (int k = 0; k < kRedZ; k++)
+                    if (k < planes) acc[k] = red_upd(op, acc[k], v[k]);
+            }
         }
-    }
+    };
+    // the largest item number of a thread's last round stays below 2^31 in the narrow form
+    const long long begin = blockIdx.x * chunk, end = begin + chunk < w.items ? begin + chunk : w.items;
+    if (w.items < (1LL << 30)) fold((unsigned)begin + threadIdx.x, (unsigned)kRedThreads, (unsigned)end);
+    else fold(begin + threadIdx.x, (long long)kRedThreads, end);
     double v = acc[0];
 #pragma unroll
     for (int k = 1; k < kRedZ; k++) v = red_comb(op, v, acc[k]);
@@ -200,27 +225,30 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce(FieldView<const double> 
 }
 
 // ---- piecewise-constant prolongation ----------------------------------------------------------
-// Fine cell p takes coarse cell floor(p / ratio). LR is log2(ratio) where that is a power of two (an
-// arithmetic shift floors like floor_div); -1 divides. Walked like the pointwise kernels; the four
-// planes' coarse and fine loads go out together. Measured (B200): AvgDown from 192^3, a copy of a 192^3
-// field and the prolongation added to it, 107 -> 67 us together with pb_stencil.cu's table kernel.
-template <int LR>
-__device__ __forceinline__ int coarse_of(int p, int ratio) { return LR >= 0 ? p >> (LR < 0 ? 0 : LR) : floor_div(p, ratio); }
+// Fine cell p takes coarse cell floor(p / ratio); a shift where the ratio is a power of two. The planes'
+// coarse and fine loads go out together. Measured (B200, us): 160^3, ratio 2 8.5, ratio 3 9.6.
+struct CoarseMap {
+    FastDiv ratio;
+    int shift;
+    int off[3], first[3];    // region coordinate p lies in source cell (p + off) / ratio + first
+};
 
-template <int LR>
-__global__ void __launch_bounds__(kWalkThreads) k_interp_const(int ratio, const double* __restrict__ src, Box3 sb,
-                                                               FieldView<double> d, Region r, Walk w, int overwrite,
+template <bool POW2>
+__global__ void __launch_bounds__(kWalkThreads) k_interp_const(FieldView<const double> s, CoarseMap m, FieldView<double> d, Walk w, int overwrite,
                                                                double scale)
 {
-    const long long Sx = bsize(sb, 0), Sxy = Sx * bsize(sb, 1);
-    walk_rows(w, [&](int x, int y, int z, int planes) {
-        const double* sq = src + (coarse_of<LR>(r.lo[0] + x, ratio) - sb.lo[0]) + Sx * (coarse_of<LR>(r.lo[1] + y, ratio) - sb.lo[1]);
+    walk_items(w, [&](int x, int y, int z, int planes) {
+        auto coarse = [&](int p, int a) {
+            const unsigned q = (unsigned)p + (unsigned)m.off[a];
+            return (int)(POW2 ? q >> m.shift : quotient(q, m.ratio)) + m.first[a];
+        };
+        const double* sq = s.p + coarse(x, 0) + s.sy * coarse(y, 1);
         double* dq = d.p + x + d.sy * y + d.sz * z;
         double v[kWalkZ], acc[kWalkZ];
 #pragma unroll
         for (int k = 0; k < kWalkZ; k++)
             if (k < planes) {
-                v[k] = __ldg(sq + Sxy * (coarse_of<LR>(r.lo[2] + z + k, ratio) - sb.lo[2]));
+                v[k] = __ldg(sq + s.sz * coarse(z + k, 2));
                 acc[k] = overwrite ? 0.0 : dq[k * d.sz];
             }
 #pragma unroll
@@ -240,7 +268,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_interp_const(int ratio, const 
 //   * a captured call's slot belongs to the graph, which may run at any time beside other reductions,
 //     and becomes idle when the graph and its executables are gone.
 struct RedSlot {
-    double* partials = nullptr;    // kRedBlocks
+    double* partials = nullptr;    // kRedBlocks, then the ticket
     unsigned int* ticket = nullptr;
     double* result = nullptr;      // allocated when a call that waits first takes the slot
     cudaEvent_t done = nullptr;    // after the last kernel (slots of streams)
@@ -374,19 +402,28 @@ static int launch_reduce(int op, const double* data, const Box3& b, const Box3& 
     Region rg;                           // an empty intersection folds nothing: the operation's initial value
     if (bempty(r)) { rg.lo[0] = b.lo[0]; rg.lo[1] = b.lo[1]; rg.lo[2] = b.lo[2]; rg.n[0] = rg.n[1] = rg.n[2] = 0; }
     else rg = region_of(r);
-    const Walk w = walk_of(rg);
-    const int rows = kRedThreads >> w.lx;
-    const long long tiles = (long long)((w.ny + rows - 1) / rows) * ((w.nz + kRedZ - 1) / kRedZ);
-    int grid = tiles < kRedBlocks ? (int)tiles : kRedBlocks;
-    if (grid < 1) grid = 1;
-    const FieldView<const double> f = view_of(data, b, rg);
+    FieldView<const double> f = view_of(data, b, rg);
+    if (rg.n[2] < kRedZ && rg.n[1] > rg.n[2]) {      // thin in z: the loads in flight go along y
+        std::swap(rg.n[1], rg.n[2]);
+        std::swap(f.sy, f.sz);
+    }
+    const bool line = rg.n[2] < kRedZ;               // thin in y as well: a thread takes kRedZ single cells
+    const Walk w = walk_of(rg, line ? 1 : kRedZ);
+    const long long blocks = (w.items + kRedThreads - 1) / kRedThreads;
+    const long long chunk = (blocks + kRedBlocks - 1) / kRedBlocks * kRedThreads;      // items of a block
+    const int grid = blocks < 1 ? 1 : (int)((w.items + chunk - 1) / chunk);
+    auto launch = [&](auto opc) {
+        constexpr int OP = decltype(opc)::value;
+        if (line) k_reduce<OP, true><<<grid, kRedThreads, 0, st>>>(f, w, chunk, s->partials, s->ticket, result);
+        else k_reduce<OP, false><<<grid, kRedThreads, 0, st>>>(f, w, chunk, s->partials, s->ticket, result);
+    };
     switch (op) {
-        case 0: k_reduce<0><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
-        case 1: k_reduce<1><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
-        case 2: k_reduce<2><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
-        case 3: k_reduce<3><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
-        case 4: k_reduce<4><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
-        default: k_reduce<5><<<grid, kRedThreads, 0, st>>>(f, w, s->partials, s->ticket, result); break;
+        case 0: launch(std::integral_constant<int, 0>{}); break;
+        case 1: launch(std::integral_constant<int, 1>{}); break;
+        case 2: launch(std::integral_constant<int, 2>{}); break;
+        case 3: launch(std::integral_constant<int, 3>{}); break;
+        case 4: launch(std::integral_constant<int, 4>{}); break;
+        default: launch(std::integral_constant<int, 5>{}); break;
     }
     PB_LAUNCH_CHECK();
     return PB_OK;
@@ -456,11 +493,12 @@ int pb_boxdata_op_f64(int op, double* dst, pb_box dst_box, const double* src, pb
     Box3 db = to_box(dst_box), sb = to_box(src_box);
     Box3 r = intersect(db, sb);
     if (bempty(r)) return PB_OK;
-    const Region rg = region_of(r);
-    const Walk w = walk_of(rg);
+    Region rg = region_of(r);
+    FieldView<double> d = view_of(dst, db, rg);
+    FieldView<const double> sv = view_of(src, sb, rg);
+    turn_thin(rg, d, sv);
+    const Walk w = walk_spread(rg);
     const dim3 grid = walk_grid(w, ncomp);
-    const FieldView<double> d = view_of(dst, db, rg);
-    const FieldView<const double> sv = view_of(src, sb, rg);
     cudaStream_t st = (cudaStream_t)stream;
     switch (op) {
         case PB_OP_ADD: k_binop<PB_OP_ADD><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), sv, bvol(sb), w, ncomp); break;
@@ -480,10 +518,11 @@ int pb_boxdata_scalar_f64(int op, double* dst, pb_box dst_box, pb_box region, do
     if (bempty(db)) return PB_ERR_BOX;
     r = bempty(r) ? db : intersect(r, db);
     if (bempty(r)) return PB_OK;
-    const Region rg = region_of(r);
-    const Walk w = walk_of(rg);
+    Region rg = region_of(r);
+    FieldView<double> d = view_of(dst, db, rg);
+    turn_thin(rg, d);
+    const Walk w = walk_spread(rg);
     const dim3 grid = walk_grid(w, ncomp);
-    const FieldView<double> d = view_of(dst, db, rg);
     cudaStream_t st = (cudaStream_t)stream;
     switch (op) {
         case PB_OP_ADD: k_scalar<PB_OP_ADD><<<grid, kWalkThreads, 0, st>>>(d, bvol(db), w, scalar, ncomp); break;
@@ -507,10 +546,12 @@ int pb_boxdata_copy_f64(const double* src, pb_box src_box, double* dst, pb_box d
     for (int d = 0; d < 3; d++) { dshift.lo[d] = db.lo[d] - sh[d]; dshift.hi[d] = db.hi[d] - sh[d]; }
     r = intersect(r, dshift);
     if (bempty(r)) return PB_OK;
-    const Region rg = region_of(r);      // source points; their destinations are shifted
-    const Walk w = walk_of(rg);
-    k_binop<PB_OP_ASSIGN><<<walk_grid(w, ncomp), kWalkThreads, 0, (cudaStream_t)stream>>>(
-        view_of(dst, db, rg, sh), bvol(db), view_of(src, sb, rg), bvol(sb), w, ncomp);
+    Region rg = region_of(r);            // source points; their destinations are shifted
+    FieldView<double> d = view_of(dst, db, rg, sh);
+    FieldView<const double> sv = view_of(src, sb, rg);
+    turn_thin(rg, d, sv);
+    const Walk w = walk_spread(rg);
+    k_binop<PB_OP_ASSIGN><<<walk_grid(w, ncomp), kWalkThreads, 0, (cudaStream_t)stream>>>(d, bvol(db), sv, bvol(sb), w, ncomp);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -522,10 +563,12 @@ int pb_forall_axpby_f64(double* out, pb_box out_box, const double* x, pb_box x_b
     Box3 ob = to_box(out_box), xb = to_box(x_box), yb = to_box(y_box);
     Box3 r = intersect(intersect(ob, xb), yb);
     if (bempty(r)) return PB_OK;
-    const Region rg = region_of(r);
-    const Walk w = walk_of(rg);
-    k_axpby<<<walk_grid(w, 1), kWalkThreads, 0, (cudaStream_t)stream>>>(view_of(out, ob, rg), view_of(x, xb, rg),
-                                                                        view_of(y, yb, rg), w, a, b);
+    Region rg = region_of(r);
+    FieldView<double> ov = view_of(out, ob, rg);
+    FieldView<const double> xv = view_of(x, xb, rg), yv = view_of(y, yb, rg);
+    turn_thin(rg, ov, xv, yv);
+    const Walk w = walk_spread(rg);
+    k_axpby<<<walk_grid(w, 1), kWalkThreads, 0, (cudaStream_t)stream>>>(ov, xv, yv, w, a, b);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -587,14 +630,25 @@ int pb_interp_constant_f64(int ratio, const double* src, pb_box src_box, double*
     rb = intersect(rb, db);
     if (bempty(rb)) return PB_OK;
     // InterpStencil::apply's final stage is "S = scale*Shift::Zeros()", folded like hostApply
-    const Region rg = region_of(rb);
-    const Walk w = walk_of(rg);
-    const dim3 grid = walk_grid(w, 1);
-    const FieldView<double> d = view_of(dst, db, rg);
+    Region rg = region_of(rb);
+    FieldView<double> d = view_of(dst, db, rg);
+    CoarseMap m;
+    m.ratio = fast_div(ratio);
+    m.shift = 31 - __builtin_clz((unsigned)ratio);
+    for (int k = 0; k < 3; k++) {
+        const int c = floor_div(rb.lo[k], ratio);
+        m.off[k] = rb.lo[k] - c * ratio;
+        m.first[k] = c - sb.lo[k];
+    }
+    FieldView<const double> sv{src, bsize(sb, 0), bsize(sb, 0) * bsize(sb, 1)};
+    if (turn_thin(rg, d, sv)) {
+        std::swap(m.off[1], m.off[2]);
+        std::swap(m.first[1], m.first[2]);
+    }
+    const Walk w = walk_spread(rg);
     cudaStream_t st = (cudaStream_t)stream;
-    if (ratio == 2) k_interp_const<1><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
-    else if (ratio == 4) k_interp_const<2><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
-    else k_interp_const<-1><<<grid, kWalkThreads, 0, st>>>(ratio, src, sb, d, rg, w, overwrite, scale);
+    if (ratio & (ratio - 1)) k_interp_const<false><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(sv, m, d, w, overwrite, scale);
+    else k_interp_const<true><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(sv, m, d, w, overwrite, scale);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }

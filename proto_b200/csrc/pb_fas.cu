@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_fas_correct(double* u, const d
 {
     const int nc = nf / 2, S = nf + 2 * kFasGhost, Sc = nc + 2 * kFasGhost;
     const long long nf2 = (long long)S * S, nc2 = (long long)nc * nc, sc2 = (long long)Sc * Sc;
-    walk_rows(w, [&](int x, int y, int z, int planes) {          // z is even: planes z, z+1 share a coarse one
+    walk_items(w, [&](int x, int y, int z, int planes) {          // z is even: planes z, z+1 share a coarse one
         double* q = u + fas_state(nf, x, y, z);
         const double* a = c0 + fas_index(nc, x / 2, y / 2, z / 2);
         const double* b = uc + fas_state(nc, x / 2, y / 2, z / 2);
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_fas_correct(double* u, const d
 __global__ void __launch_bounds__(kWalkThreads) k_fas_pack(const double* __restrict__ src, double* u, int n, Walk w)
 {
     const long long S = n + 2 * kFasGhost;
-    walk_rows(w, [&](int x, int y, int z, int planes) {          // x, y of the grown plane
+    walk_items(w, [&](int x, int y, int z, int planes) {          // x, y of the grown plane
         const double* q = src + lap4_wrap(x - kFasGhost, n) + (long long)n * (lap4_wrap(y - kFasGhost, n) + (long long)n * z);
         double* o = u + x + S * (y + S * z);
         double v[kWalkZ];
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_fas_pack(const double* __restr
 __global__ void __launch_bounds__(kWalkThreads) k_fas_unpack(const double* __restrict__ u, double* dst, int n, Walk w)
 {
     const long long S = n + 2 * kFasGhost;
-    walk_rows(w, [&](int x, int y, int z, int planes) {
+    walk_items(w, [&](int x, int y, int z, int planes) {
         double v[kWalkZ];
 #pragma unroll
         for (int k = 0; k < kWalkZ; k++)

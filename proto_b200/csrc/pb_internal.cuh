@@ -124,7 +124,7 @@ __device__ __forceinline__ float squot(float a, float b) { return __fdividef(a, 
 // Reduction<T,Abs>::update (Proto_ReductionImplem.H:87): NaN inputs leave the value unchanged.
 __device__ __forceinline__ double upd_abs(double v1, double v2)
 {
-    double a = v2 > 0 ? v2 : -v2;
+    const double a = fabs(v2);
     return (v1 < a) ? a : v1;
 }
 // atomic max of a non-negative double through its bit pattern (monotone for x >= 0)

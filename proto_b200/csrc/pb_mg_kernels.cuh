@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_relax_first(const T* __restric
                                                               T* out, RelaxCoef<T> k, Walk w)
 {
     const int n = k.n;
-    walk_rows(w, [&](int x, int y, int z, int planes) {
+    walk_items(w, [&](int x, int y, int z, int planes) {
         const long long i = x + (long long)n * (y + (long long)n * z), n2 = (long long)n * n;
         T rho[kWalkZ], al[kWalkZ];
 #pragma unroll
@@ -813,7 +813,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_pack_in(const T* __restrict__ 
 {
     const long long Sz = (long long)sx * (n + 2), n2 = (long long)n * n;
     auto wrap = [&](int c) { return c == 0 ? n - 1 : (c > n ? 0 : c - 1); };   // grown coordinate -> valid cell
-    walk_rows(w, [&](int x, int y, int z, int planes) {
+    walk_items(w, [&](int x, int y, int z, int planes) {
         const T* q = src + wrap(x) + (long long)n * wrap(y);
         T v[kWalkZ];
 #pragma unroll
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_pack_in(const T* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(kWalkThreads) k_pack_out(const T* __restrict__ g, T* dst, int n, int sx, Walk w)
 {
-    walk_rows(w, [&](int x, int y, int z, int planes) {
+    walk_items(w, [&](int x, int y, int z, int planes) {
         T v[kWalkZ];
 #pragma unroll
         for (int k = 0; k < kWalkZ; k++)

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ sr
     for (int c = blockIdx.z; c < a.ncomp; c += gridDim.z) {
         const T* sp = src + c * a.svol;
         T* dp = dst + c * a.dvol;
-        walk_rows(w, [&](int x, int y, int z, int planes) {
+        walk_items(w, [&](int x, int y, int z, int planes) {
             I at[kWalkZ];
             T acc[kWalkZ];
             T* dq = dp + a.dx * x + a.dy * y + a.dz * z;
@@ -149,17 +149,18 @@ template <typename T>
 struct CubeArgs {
     T c[27];                    // by cube position (z+1)*9 + (y+1)*3 + (x+1)
     int ncomp, init_zero, zd, chunks;
+    int nx, ny, nz, lx;         // lx: log2 of the lanes along x
     long long svol, dvol;
 };
 template <typename T, bool CORNERS>
 __global__ void __launch_bounds__(kCubeThreads, kCubePerSm) k_cube(FieldView<const T> s, FieldView<T> d,
-                                                                   const __grid_constant__ CubeArgs<T> a, Walk w)
+                                                                   const __grid_constant__ CubeArgs<T> a)
 {
-    const int lane = threadIdx.x & ((1 << w.lx) - 1), row = threadIdx.x >> w.lx;
-    const int x = blockIdx.x * (1 << w.lx) + lane, y = blockIdx.y * (kCubeThreads >> w.lx) + row;
-    if (x >= w.nx || y >= w.ny) return;
+    const int lane = threadIdx.x & ((1 << a.lx) - 1), row = threadIdx.x >> a.lx;
+    const int x = blockIdx.x * (1 << a.lx) + lane, y = blockIdx.y * (kCubeThreads >> a.lx) + row;
+    if (x >= a.nx || y >= a.ny) return;
     for (int u = blockIdx.z; u < a.chunks * a.ncomp; u += gridDim.z) {
-        const int comp = u / a.chunks, z0 = (u - comp * a.chunks) * a.zd, z1 = min(z0 + a.zd, w.nz);
+        const int comp = u / a.chunks, z0 = (u - comp * a.chunks) * a.zd, z1 = min(z0 + a.zd, a.nz);
         const T* q = s.p + comp * a.svol + x + s.sy * y + s.sz * (z0 - 1);   // the next plane to load
         T* o = d.p + comp * a.dvol + x + d.sy * y + d.sz * z0;               // the next cell to start
         auto load = [&](T* p) {
@@ -412,12 +413,19 @@ static int launch_table(const pb_stencil* s, const T* src, const Box3& sb, T* ds
     return PB_OK;
 }
 
+// log2 of the column kernel's lanes along x: short rows take more rows per block, with fewer idle lanes
+static int cube_lanes(long long nx)
+{
+    int lx = 5;
+    while (lx > 3 && (1 << (lx - 1)) >= nx) lx--;
+    return lx;
+}
+
 template <typename T>
 static int launch_cube(const pb_stencil* s, const T* src, const Box3& sb, T* dst, const Box3& db, const Box3& ib,
                        int ncomp, int init_to_zero, T scale, cudaStream_t st)
 {
     const Region rg = region_of(ib);
-    const Walk w = walk_of(rg);
     CubeArgs<T> a{};
     a.ncomp = ncomp;
     a.init_zero = init_to_zero ? 1 : 0;
@@ -425,26 +433,30 @@ static int launch_cube(const pb_stencil* s, const T* src, const Box3& sb, T* dst
     a.dvol = bvol(db);
     for (int j = 0; j < (int)s->coefs.size(); j++)
         a.c[(s->offs[3 * j + 2] + 1) * 9 + (s->offs[3 * j + 1] + 1) * 3 + s->offs[3 * j] + 1] = fold<T>(s->coefs[j], scale);
-    const int rows = kCubeThreads >> w.lx, gx = (w.nx + (1 << w.lx) - 1) >> w.lx, gy = (w.ny + rows - 1) / rows;
+    a.nx = rg.n[0];
+    a.ny = rg.n[1];
+    a.nz = rg.n[2];
+    a.lx = cube_lanes(a.nx);
+    const int rows = kCubeThreads >> a.lx, gx = (a.nx + (1 << a.lx) - 1) >> a.lx, gy = (a.ny + rows - 1) / rows;
     // the z chunk that makes waves of resident blocks x (planes + 2) smallest: a chunk starts with two
     // planes of loads beyond its own
     const long long slots = (long long)kCubePerSm * cached_sm_count();
     long long best = -1;
-    for (int zd = 4; zd < w.nz + 4; zd += zd < 64 ? 4 : 16) {
-        const long long blocks = (long long)gx * gy * ((w.nz + zd - 1) / zd) * ncomp;
+    for (int zd = 4; zd < a.nz + 4; zd += zd < 64 ? 4 : 16) {
+        const long long blocks = (long long)gx * gy * ((a.nz + zd - 1) / zd) * ncomp;
         const long long cost = (blocks + slots - 1) / slots * (zd + 2);
         if (best < 0 || cost < best) {
             best = cost;
             a.zd = zd;
         }
     }
-    a.chunks = (w.nz + a.zd - 1) / a.zd;
+    a.chunks = (a.nz + a.zd - 1) / a.zd;
     const long long gz = (long long)a.chunks * ncomp;
     const dim3 grid(gx, gy, (unsigned)(gz < 65535 ? gz : 65535));
     const FieldView<const T> sv = view_of(src, sb, rg);
     const FieldView<T> dv = view_of(dst, db, rg);
-    if (s->cube == 27) k_cube<T, true><<<grid, kCubeThreads, 0, st>>>(sv, dv, a, w);
-    else k_cube<T, false><<<grid, kCubeThreads, 0, st>>>(sv, dv, a, w);
+    if (s->cube == 27) k_cube<T, true><<<grid, kCubeThreads, 0, st>>>(sv, dv, a);
+    else k_cube<T, false><<<grid, kCubeThreads, 0, st>>>(sv, dv, a);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
