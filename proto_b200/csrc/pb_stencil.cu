@@ -87,10 +87,12 @@ int encode_tmap_3d(CUtensorMap* map, const void* base, int esize, long long Sx, 
 // ---- generic table kernel ---------------------------------------------------------------------
 // Any table: acc = sum_j c_j * src[first + off_j], first the term of the span's low corner, so every
 // offset is non-negative and, with at most 2^32 source cells, 32 bits wide: a term is then one load
-// from a uniform base plus the thread's 32-bit index, one multiply and one add. A thread takes kWalkZ
-// planes of a point, so a term's coefficient and offset are read once for four cells and four to
-// sixteen loads are in flight (one cell per thread with 64-bit offsets issued about seven
-// instructions per term). Bound by the issue of the terms' loads.
+// from a uniform base plus the thread's 32-bit index, one multiply and one add; eight terms' loads are in
+// flight. A thread takes one cell: with four planes a thread a small box has a quarter of the warps to
+// hide its chain of loads, and a block's source lines outgrow L1 between the two halves of a ratio-2 row.
+// Bound by the issue of the terms' loads. Measured (B200, us, one cell a thread / four): 27 points on 33^3
+// 3.2 / 7.4, AvgDown to 64^3 3.4 / 4.8, to 160^3 43 / 69, 64 terms on 160^3 56 / 61.
+constexpr int kTableTerms = 8;    // unroll of the term loop
 template <typename T, typename I, int NMAX>
 struct TableKernelArgs {
     T c[NMAX];
@@ -107,27 +109,13 @@ __global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ sr
     for (int c = blockIdx.z; c < a.ncomp; c += gridDim.z) {
         const T* sp = src + c * a.svol;
         T* dp = dst + c * a.dvol;
-        walk_items(w, [&](int x, int y, int z, int planes) {
-            I at[kWalkZ];
-            T acc[kWalkZ];
+        walk_items(w, [&](int x, int y, int z, int) {
             T* dq = dp + a.dx * x + a.dy * y + a.dz * z;
-            at[0] = (I)(a.sx * x + a.sy * y + a.sz * z);
-#pragma unroll
-            for (int k = 1; k < kWalkZ; k++) at[k] = k < planes ? (I)(at[k - 1] + (I)a.sz) : at[0];
-#pragma unroll
-            for (int k = 0; k < kWalkZ; k++) acc[k] = a.init_zero || k >= planes ? T(0) : dq[k * a.dz];
-#pragma unroll 4
-            for (int j = 0; j < a.n; j++) {
-                const T* sj = sp + a.off[j];
-                T v[kWalkZ];
-#pragma unroll
-                for (int k = 0; k < kWalkZ; k++) v[k] = __ldg(sj + at[k]);
-#pragma unroll
-                for (int k = 0; k < kWalkZ; k++) acc[k] = dadd(acc[k], dmul(a.c[j], v[k]));
-            }
-#pragma unroll
-            for (int k = 0; k < kWalkZ; k++)
-                if (k < planes) dq[k * a.dz] = acc[k];
+            const I at = (I)(a.sx * x + a.sy * y + a.sz * z);
+            T acc = a.init_zero ? T(0) : *dq;
+#pragma unroll kTableTerms
+            for (int j = 0; j < a.n; j++) acc = dadd(acc, dmul(a.c[j], __ldg(sp + a.off[j] + at)));
+            *dq = acc;
         });
     }
 }
@@ -140,9 +128,11 @@ __global__ void __launch_bounds__(kWalkThreads) k_table(const T* __restrict__ sr
 // registers. Bound by FP64 issue (27 multiplies and 27 adds, each rounded: 12 us at 3.95 M cells) and
 // load latency. Measured (B200, two components of 193 x 161 x 127 FP64 cells): 68 us a component one cell
 // per thread, 43 with the three planes held, 33 with the next plane loaded a step early, 28 with four more
-// asked into L2. Below kCubeMin cells the columns are too few to fill the GPU, and the table kernel takes
-// four cells per thread.
-constexpr long long kCubeMin = 1 << 17;
+// asked into L2. Below kCubeMin cells the columns are too few to fill the GPU (16^3: 2.88 us, table 2.84;
+// 24^3 2.84 / 3.15; 33^3 2.95 / 3.23), and boxes thin along an axis leave its threads idle (share of steps
+// that give a cell: 256 x 256 x 2 0.5, 3.1 / 4.1; 2048 x 2048 x 1 0.33, 78 / 57; 2 x 1024 x 1024 0.25, 45 / 30).
+constexpr long long kCubeMin = 1 << 15;
+constexpr double kCubeShare = 0.4;
 constexpr int kCubeThreads = 128, kCubePerSm = 5;
 constexpr int kCubePrefetch = 4;   // planes past the next one whose lines are asked into L2
 template <typename T>
@@ -382,7 +372,7 @@ static int launch_table(const pb_stencil* s, const T* src, const Box3& sb, T* ds
                         int ncomp, int init_to_zero, T scale, int n, cudaStream_t st)
 {
     const Region rg = region_of(ib);
-    const Walk w = walk_of(rg);
+    const Walk w = walk_of(rg, 1);
     const long long sS[3] = {1, bsize(sb, 0), bsize(sb, 0) * bsize(sb, 1)};
     const long long dS[3] = {1, bsize(db, 0), bsize(db, 0) * bsize(db, 1)};
     TableKernelArgs<T, I, NMAX> a;
@@ -419,6 +409,14 @@ static int cube_lanes(long long nx)
     int lx = 5;
     while (lx > 3 && (1 << (lx - 1)) >= nx) lx--;
     return lx;
+}
+// share of the column kernel's thread steps that give a cell (a column starts with two planes of loads)
+static double cube_share(const Box3& b)
+{
+    const long long n[3] = {bsize(b, 0), bsize(b, 1), bsize(b, 2)};
+    const int lx = cube_lanes(n[0]), lanes = 1 << lx, rows = kCubeThreads >> lx;
+    auto full = [](long long v, int m) { return (double)v / (double)((v + m - 1) / m * m); };
+    return full(n[0], lanes) * full(n[1], rows) * n[2] / (n[2] + 2.0);
 }
 
 template <typename T>
@@ -500,7 +498,7 @@ static int apply_impl(const pb_stencil* s, const T* src, pb_box src_box, T* dst,
     if (n > kMaxTerms) return PB_ERR_UNSUPPORTED;
     ib = clip_to_dst(s, ib, db);
     if (bempty(ib)) return PB_OK;
-    if (s->cube && bvol(ib) >= kCubeMin && (bsize(ib, 1) + 3) / 4 <= 65535)
+    if (s->cube && bvol(ib) >= kCubeMin && cube_share(ib) >= kCubeShare && (bsize(ib, 1) + 3) / 4 <= 65535)
         return launch_cube<T>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, st);
     if (svol > 0xffffffffLL) return launch_table<T, long long, kMaxTerms>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
     if (n <= 32) return launch_table<T, unsigned, 32>(s, src, sb, dst, db, ib, ncomp, init_to_zero, scale, n, st);
