@@ -87,6 +87,22 @@ __device__ __forceinline__ void lap4_cells(const Lap4Taps& n, const double (&wm)
     }
 }
 
+// t of a cell by itself, from its values at -2, -1, +1, +2 along each axis
+__device__ __forceinline__ double lap4_cell(const double (&v)[3][4], double c, const FasCoef& k)
+{
+    double div = 0.0;
+    const double B = dmul(k.g[1], c);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const double m2 = v[d][0], m1 = v[d][1], p1 = v[d][2], p2 = v[d][3];
+        const double Fp = dmul(k.cp, dsub(dsub(dadd(dmul(k.g[0], m1), B), dmul(k.g[1], p1)), dmul(k.g[0], p2)));
+        const double Fm = dmul(k.cp, dsub(dsub(dadd(dmul(k.g[0], m2), dmul(k.g[1], m1)), B), dmul(k.g[0], p1)));
+        div = d == 0 ? Fp : dadd(div, Fp);
+        div = dsub(div, Fm);
+    }
+    return dadd(0.0, div);
+}
+
 // The epilogue: cursor(x, y, z0, act0, act1) once per thread (its addresses at the chunk's first plane);
 // per plane pre(cursor, ahead, p0, p1) loads what it needs of both cells, `ahead` planes above the cursor,
 // cells(cursor, z, t0, t1, c0, c1, p0, p1) takes the rows' t and centre values (every thread of the block

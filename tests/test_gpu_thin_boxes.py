@@ -123,7 +123,7 @@ def _us(f, calls=10):
     return best
 
 
-@pytest.mark.parametrize("name", ["add", "copy", "interp3", "reduce", "laplacian27"])
+@pytest.mark.parametrize("name", ["add", "copy", "interp3", "reduce", "laplacian27", "boxop"])
 def test_a_line_costs_what_a_solid_box_does(golden, pb, name):
     """The same 2^18 cells as a 64^3 box and as lines along each axis. The bound is loose: a line reads up to 25
     times the source of a solid box's stencil. A kernel that leaves lanes or blocks idle on lines takes 20
