@@ -16,6 +16,7 @@
 
 #include "pb_internal.cuh"
 #include "pb_stencil_impl.cuh"
+#include "pb_walk.cuh"
 
 namespace pb {
 
@@ -30,36 +31,33 @@ struct MotionItem {
 
 // A unit of exchange work: up to kUnitCells consecutive cells (x fastest) of one item's region, the
 // first at region coordinates (x, y, z). A region is 8 cells at a corner and thousands on a face, so
-// a warp per unit balances them; each lane keeps kUnitCells / 32 loads in flight. Bound by the ghost
-// cells' bytes (the x faces move 16-byte pieces of 32-byte sectors) and memory latency. Measured (B200,
-// 1498 items of 2 ghost cells): 29.8 -> 12.4 us against one block per item with one cell per thread and
-// 64-bit divisions.
+// a warp per unit balances them; each lane keeps kUnitCells / 32 loads in flight. A unit holds all that
+// its warp needs (one round of loads before the cells', not one for the unit and one for its item). Bound
+// by the ghost cells' bytes (the x faces move 16-byte pieces of 32-byte sectors) and memory latency.
 constexpr int kUnitCells = 256;
 struct ExchangeUnit {
-    int item;
-    int x, y, z;
-    int count;
+    long long src, dst;        // slab offsets of region coordinate (0, 0, 0), component 0
+    long long svol, dvol;      // component strides
+    int sSx, sSy, dSx, dSy;    // extents of the grown boxes
+    int x, y, z, count;
+    FastDiv nx, ny;            // the region's extents
 };
 
-__global__ void __launch_bounds__(256) k_exchange(double* slab, const MotionItem* __restrict__ items,
-                                                  const ExchangeUnit* __restrict__ units, int nunits, int ncomp)
+__global__ void __launch_bounds__(256) k_exchange(double* slab, const ExchangeUnit* __restrict__ units, int nunits, int ncomp)
 {
     const int u = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (u >= nunits) return;
     const ExchangeUnit un = units[u];
-    const MotionItem& it = items[un.item];
     constexpr int K = kUnitCells / 32;
-    const unsigned nx = it.rn[0], ny = it.rn[1];
-    const long long dSx = it.dS[0], dSxy = dSx * it.dS[1], sSx = it.sS[0], sSxy = sSx * it.sS[1];
-    // region coordinate (0, 0, 0) in the destination and in the source
-    double* d0 = slab + it.dOff + (it.rlo[0] - it.dlo[0]) + dSx * (it.rlo[1] - it.dlo[1]) + dSxy * (it.rlo[2] - it.dlo[2]);
-    const double* s0 = slab + it.sOff + (it.rlo[0] - it.sh[0] - it.slo[0]) + sSx * (it.rlo[1] - it.sh[1] - it.slo[1]) +
-                       sSxy * (it.rlo[2] - it.sh[2] - it.slo[2]);
+    const long long dSx = un.dSx, dSxy = dSx * un.dSy, sSx = un.sSx, sSxy = sSx * un.sSy;
+    double* d0 = slab + un.dst;
+    const double* s0 = slab + un.src;
     long long di[K], si[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        const unsigned px = un.x + lane + 32 * k, qy = px / nx, py = un.y + qy, qz = py / ny;
-        const long long x = px - qy * nx, y = py - qz * ny, z = un.z + qz;
+        if (32 * k >= un.count) break;         // the whole warp: small regions pay for their own cells
+        const unsigned px = un.x + lane + 32 * k, qy = quotient(px, un.nx), py = un.y + qy, qz = quotient(py, un.ny);
+        const long long x = px - qy * un.nx.d, y = py - qz * un.ny.d, z = un.z + qz;
         di[k] = x + dSx * y + dSxy * z;
         si[k] = x + sSx * y + sSxy * z;
     }
@@ -67,10 +65,10 @@ __global__ void __launch_bounds__(256) k_exchange(double* slab, const MotionItem
         double v[K];
 #pragma unroll
         for (int k = 0; k < K; k++)
-            if (lane + 32 * k < un.count) v[k] = s0[c * it.svol + si[k]];
+            if (lane + 32 * k < un.count) v[k] = s0[c * un.svol + si[k]];
 #pragma unroll
         for (int k = 0; k < K; k++)
-            if (lane + 32 * k < un.count) d0[c * it.dvol + di[k]] = v[k];
+            if (lane + 32 * k < un.count) d0[c * un.dvol + di[k]] = v[k];
     }
 }
 
@@ -555,7 +553,6 @@ struct pb_level {
     std::vector<long long> offsets;
     long long slab_elems;
     std::vector<pb::MotionItem> items;
-    pb::MotionItem* d_items = nullptr;
     std::vector<pb::ExchangeUnit> units;       // the items' regions in warp-sized pieces
     pb::ExchangeUnit* d_units = nullptr;
     std::vector<pb::PatchTile> tiles;          // one cell per thread
@@ -629,12 +626,27 @@ static void build_items(pb_level* lv)
 
 static void build_units(pb_level* lv)
 {
-    for (int i = 0; i < (int)lv->items.size(); i++) {
-        const MotionItem& m = lv->items[i];
+    for (const MotionItem& m : lv->items) {
         const long long nx = m.rn[0], ny = m.rn[1], vol = nx * ny * m.rn[2];
-        for (long long f = 0; f < vol; f += kUnitCells)
-            lv->units.push_back(ExchangeUnit{i, (int)(f % nx), (int)(f / nx % ny), (int)(f / (nx * ny)),
-                                             (int)std::min<long long>(kUnitCells, vol - f)});
+        ExchangeUnit un;
+        un.dst = m.dOff + (m.rlo[0] - m.dlo[0]) + m.dS[0] * ((m.rlo[1] - m.dlo[1]) + (long long)m.dS[1] * (m.rlo[2] - m.dlo[2]));
+        un.src = m.sOff + (m.rlo[0] - m.sh[0] - m.slo[0]) +
+                 m.sS[0] * ((m.rlo[1] - m.sh[1] - m.slo[1]) + (long long)m.sS[1] * (m.rlo[2] - m.sh[2] - m.slo[2]));
+        un.dvol = m.dvol;
+        un.svol = m.svol;
+        un.dSx = m.dS[0];
+        un.dSy = m.dS[1];
+        un.sSx = m.sS[0];
+        un.sSy = m.sS[1];
+        un.nx = fast_div(m.rn[0]);
+        un.ny = fast_div(m.rn[1]);
+        for (long long f = 0; f < vol; f += kUnitCells) {
+            un.x = (int)(f % nx);
+            un.y = (int)(f / nx % ny);
+            un.z = (int)(f / (nx * ny));
+            un.count = (int)std::min<long long>(kUnitCells, vol - f);
+            lv->units.push_back(un);
+        }
     }
 }
 
@@ -642,7 +654,7 @@ static int launch_exchange(const pb_level* lv, double* slab, cudaStream_t st)
 {
     const int nu = (int)lv->units.size();
     if (nu == 0) return PB_OK;
-    k_exchange<<<(nu + 7) / 8, 256, 0, st>>>(slab, lv->d_items, lv->d_units, nu, lv->ncomp);
+    k_exchange<<<(nu + 7) / 8, 256, 0, st>>>(slab, lv->d_units, nu, lv->ncomp);
     PB_LAUNCH_CHECK();
     return PB_OK;
 }
@@ -935,20 +947,15 @@ int pb_level_create(const pb_box* patches, int npatch, const int ghost[3], pb_bo
     if (lv->pair_ok) build_tiles(lv, 2);
     cudaGetDevice(&lv->device);
     if (!lv->items.empty()) {
-        if (cudaMalloc(&lv->d_items, lv->items.size() * sizeof(MotionItem)) != cudaSuccess ||
-            cudaMemcpy(lv->d_items, lv->items.data(), lv->items.size() * sizeof(MotionItem), cudaMemcpyHostToDevice) !=
-                cudaSuccess ||
-            cudaMalloc(&lv->d_units, lv->units.size() * sizeof(ExchangeUnit)) != cudaSuccess ||
+        if (cudaMalloc(&lv->d_units, lv->units.size() * sizeof(ExchangeUnit)) != cudaSuccess ||
             cudaMemcpy(lv->d_units, lv->units.data(), lv->units.size() * sizeof(ExchangeUnit), cudaMemcpyHostToDevice) !=
                 cudaSuccess) {
-            cudaFree(lv->d_items);
             cudaFree(lv->d_units);
             delete lv;
             return PB_ERR_CUDA;
         }
     }
     if (upload_tiles(lv) != PB_OK || upload_tiles(lv, 2) != PB_OK) {
-        cudaFree(lv->d_items);
         cudaFree(lv->d_units);
         cudaFree(lv->d_tiles);
         delete lv;
@@ -962,7 +969,6 @@ int pb_level_destroy(pb_level* lv)
 {
     if (!lv) return PB_OK;
     drop_graph(lv);
-    cudaFree(lv->d_items);
     cudaFree(lv->d_units);
     cudaFree(lv->d_tiles);
     cudaFree(lv->d_tiles2);

@@ -231,3 +231,23 @@ def test_pair_steps_at_odd_y_extents(golden, pb, epilogue, tune):
     pb.device_check()
     # an odd number of steps: the result is in the first slab either way
     assert np.array_equal(_valid(lv, a.cpu().numpy()), _valid(lv, a2.cpu().numpy()))
+
+
+@pytest.mark.parametrize("widths,g,ncomp", [([[3, 5], [4], [7, 2]], (2, 1, 2), 1), ([[17, 3], [9, 24], [13]], (3, 2, 0), 2),
+                                            ([[40], [33, 7], [21, 30]], (2, 2, 2), 3)])
+def test_exchange_of_components_and_ragged_regions(pb, port, widths, g, ncomp):
+    """Regions of a few cells, and regions that leave the last unit part filled; per-axis ghost widths."""
+    import torch
+    boxes, L = W.amr_patches(widths)
+    dom = ((0, 0, 0), [v - 1 for v in L])
+    lv = pb.Level([pb.Box(*b) for b in boxes], g, pb.Box(*dom), (1, 0, 1), ncomp=ncomp)
+    size = [ncomp * int(np.prod([p.size(d) + 2 * g[d] for d in range(3)])) for p in lv.patches]
+    host = np.random.default_rng(sum(L)).uniform(-1, 1, max(o + n for o, n in zip(lv.offsets, size)))
+    slab = torch.from_numpy(host.copy()).cuda()
+    lv.exchange(slab)
+    torch.cuda.synchronize()
+    datas = [host[o:o + n].copy() for o, n in zip(lv.offsets, size)]
+    port.exchange([b[0] + b[1] for b in boxes], g, dom, (1, 0, 1), datas, ncomp)
+    got = slab.cpu().numpy()
+    for o, n, d in zip(lv.offsets, size, datas):
+        assert np.array_equal(got[o:o + n], d)
