@@ -371,18 +371,20 @@ __global__ void __launch_bounds__(kLevelThreads) k_level_star_tiled(const double
 // (four cells, a CTA of 128 threads), so that the rows share their y taps and the staging, the barrier
 // and the loop's bookkeeping are paid once for four cells. Bound by instruction issue and the planes'
 // latency. Measured (B200, 512 patches, 21 M cells): 106.6 us a step with one row per thread, 102.6 with
-// two. Same terms in the same order per cell, so bitwise the one-cell paths.
+// two. A small level's tiles are all resident at once and the step takes as long as one CTA: there a
+// thread takes one row (ROWS = 1, 256 threads). Measured (us a step, one row / two): 8 patches of 8^3 4.4 /
+// 6.1, one of 64^3 8.1 / 9.9, 512 of 8^3 8.0 / 8.5, 512 of 16^3 (2.1 M cells) 17.06 / 17.07, 16 M cells 76.6 /
+// 74.7. Same terms in the same order per cell, so bitwise the one-cell paths.
 constexpr int kLevelPairPlaneMax = (64 + 4) * (8 + 4);   // (2tx+4)(ty+4) <= 816 for tx in {8, 16, 32}
-constexpr int kLevelPairThreads = kLevelThreads / 2;      // two rows each
 
-template <class S>
-__global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const double* __restrict__ u, double* out,
+template <class S, int ROWS>
+__global__ void __launch_bounds__(kLevelThreads / ROWS, ROWS == 2 ? 5 : 4) k_level_star_pair(const double* __restrict__ u, double* out,
                                                                    const PatchTile* __restrict__ tiles,
                                                                    Coefs<double> cf, double a, int euler)
 {
     // ring of Q = 2R+1 planes, lead L = Q-1: the z loop is unrolled by Q so ring slots and the
     // register window's slots are compile-time constants at every step (no window moves)
-    constexpr int R = S::R, W = 2 * R + 1, Q = W, L = Q - 1, PM = kLevelPairPlaneMax;
+    constexpr int R = S::R, W = 2 * R + 1, Q = W, L = Q - 1, PM = kLevelPairPlaneMax, NT = kLevelThreads / ROWS;
     static_assert(R == 2, "cell pairs line up with 16-byte boundaries for a halo of 2");
     __shared__ __align__(16) double ring[Q * PM];
     const PatchTile t = tiles[blockIdx.x];
@@ -392,16 +394,16 @@ __global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const 
     const int g0 = t.gh[0], g1 = t.gh[1], g2 = t.gh[2];
     const long long Sx = t.gS[0], Sy = t.gS[1], Sxy = Sx * Sy;
     const int lx = threadIdx.x % tx, ly = threadIdx.x / tx;
-    const int x = t.x0 + 2 * lx, y = t.y0 + 2 * ly;
-    const bool act = x < nx && y < ny, act1 = act && y + 1 < ny;
+    const int x = t.x0 + 2 * lx, y = t.y0 + ROWS * ly;
+    const bool act = x < nx && y < ny, act1 = ROWS == 2 && act && y + 1 < ny;
     const int z0 = t.z0, z1 = min(t.z0 + t.zd, nz);
-    constexpr int kMaxLoads = (PM / 2 + kLevelPairThreads - 1) / kLevelPairThreads;
+    constexpr int kMaxLoads = (PM / 2 + NT - 1) / NT;
     const double* lp[kMaxLoads];
     long long ls[kMaxLoads];
     bool lv_[kMaxLoads];
 #pragma unroll
     for (int k = 0; k < kMaxLoads; k++) {
-        const int i = threadIdx.x + k * kLevelPairThreads;   // pair index in the staged tile
+        const int i = threadIdx.x + k * NT;   // pair index in the staged tile
         const int hx = i % PX, hy = i / PX;
         const int xx = t.x0 - R + 2 * hx, yy = t.y0 - R + hy;
         const bool xo = xx < 0 || xx >= nx, yo = yy < 0 || yy >= ny;
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const 
 #pragma unroll
             for (int k = 0; k < kMaxLoads; k++)
                 if (lv_[k]) {
-                    cp_async16(ring0 + 8u * (q * PM + 2 * k * kLevelPairThreads), lp[k]);
+                    cp_async16(ring0 + 8u * (q * PM + 2 * k * NT), lp[k]);
                     lp[k] += ls[k];
                 }
         }
@@ -457,24 +459,24 @@ __global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const 
 #pragma unroll
     for (int k = 0; k < L; k++) stage(z0 + k, k);
     // window slot of plane p: (p - z0 + R) mod W
-    double2 w[2][W];
+    double2 w[ROWS][W];
     if (act) {
 #pragma unroll
         for (int k = 0; k < 2 * R; k++)
 #pragma unroll
-            for (int r = 0; r < 2; r++) w[r][k] = zcol(z0 - R + k, r);
+            for (int r = 0; r < ROWS; r++) w[r][k] = zcol(z0 - R + k, r);
     }
     // The last row of a patch of odd y extent has no second row: row y + 1, its +y tap, is the next patch's
     // first. From plane z0 + R on the ring holds it; the planes before come from that patch here.
-    if (act && !act1) {
+    if (ROWS == 2 && act && !act1) {
         const long long Sq = t.nb_S[1][1];
         const double* q = u + t.nb_off[1][1] + (x + g0) + Sx * (g1 + Sq * (z0 + g2));
 #pragma unroll
         for (int k = 0; k < R; k++)
-            if (z0 + k < z1) w[1][R + k] = __ldg(reinterpret_cast<const double2*>(q + Sx * Sq * k));
+            if (z0 + k < z1) w[ROWS - 1][R + k] = __ldg(reinterpret_cast<const double2*>(q + Sx * Sq * k));
     }
     double* op = out + t.off + cxy + Sxy * t.z0;
-    const int sc = (2 * ly + R) * BX + (2 * lx + R);   // even: pairs are 16-byte aligned in the ring
+    const int sc = (ROWS * ly + R) * BX + (2 * lx + R);   // even: pairs are 16-byte aligned in the ring
     auto ring2 = [&](const double* q) { return *reinterpret_cast<const double2*>(q); };
     // one plane; J = (z - z0) mod Q, so plane z sits in ring slot J and window slot J + R
     auto step = [&](auto Jc, int z) {
@@ -486,12 +488,14 @@ __global__ void __launch_bounds__(kLevelPairThreads, 5) k_level_star_pair(const 
             constexpr int qr = (J + R) % Q, wn = (J + 2 * R) % W, wc = (J + R) % W;
             const bool in = z + R < z1;
 #pragma unroll
-            for (int r = 0; r < 2; r++) w[r][wn] = in ? ring2(ring + qr * PM + sc + r * BX) : zcol(z + R, r);
+            for (int r = 0; r < ROWS; r++) w[r][wn] = in ? ring2(ring + qr * PM + sc + r * BX) : zcol(z + R, r);
             const double* pl = ring + J * PM + sc;
-            // rows y-2, y-1, y, y+1, y+2, y+3 of this pair
-            const double2 yy[6] = {ring2(pl - 2 * BX), ring2(pl - BX), w[0][wc], w[1][wc], ring2(pl + 2 * BX), ring2(pl + 3 * BX)};
+            // rows y-2 .. y+ROWS+1 of this pair
+            double2 yy[4 + ROWS];
 #pragma unroll
-            for (int r = 0; r < 2; r++) {
+            for (int r = 0; r < 4 + ROWS; r++) yy[r] = r < 2 || r >= 2 + ROWS ? ring2(pl + (r - 2) * BX) : w[r < 2 ? 0 : r - 2 < ROWS ? r - 2 : 0][wc];
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) {
                 const double2 xm = ring2(pl + r * BX - 2);   // x-2, x-1
                 const double2 xc = w[r][wc];                 // x, x+1
                 const double2 xp = ring2(pl + r * BX + 2);   // x+2, x+3
@@ -552,6 +556,7 @@ struct pb_level {
     int ncomp;
     std::vector<long long> offsets;
     long long slab_elems;
+    long long cells = 0;                       // valid cells of one component
     std::vector<pb::MotionItem> items;
     std::vector<pb::ExchangeUnit> units;       // the items' regions in warp-sized pieces
     pb::ExchangeUnit* d_units = nullptr;
@@ -808,7 +813,9 @@ static int launch_level_star(const pb_level* lv, int shape, const double* u, dou
     if (fused && !lv->tensor) return PB_ERR_ARG;
     if (use_pairs(lv, shape, fused, u, out)) {
         const unsigned np = (unsigned)lv->tiles2.size();
-        if (np) k_level_star_pair<ShapeLap13><<<np, kLevelPairThreads, 0, st>>>(u, out, lv->d_tiles2, cf, a, euler);
+        // as many cells as four full tiles of 32 x 16 x 16 per SM
+        if (lv->cells > 4LL * 8192 * cached_sm_count() && np) k_level_star_pair<ShapeLap13, 2><<<np, kLevelThreads / 2, 0, st>>>(u, out, lv->d_tiles2, cf, a, euler);
+        else if (np) k_level_star_pair<ShapeLap13, 1><<<np, kLevelThreads, 0, st>>>(u, out, lv->d_tiles2, cf, a, euler);
         PB_LAUNCH_CHECK();
         return PB_OK;
     }
@@ -937,6 +944,7 @@ int pb_level_create(const pb_box* patches, int npatch, const int ghost[3], pb_bo
         off += gv * ncomp;
         off = (off + 31) / 32 * 32;   // every patch starts 256-byte aligned
     }
+    for (const Box3& b : lv->patches) lv->cells += bvol(b);
     lv->slab_elems = off;
     build_items(lv);
     build_units(lv);

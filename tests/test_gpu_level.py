@@ -209,12 +209,14 @@ def test_fused_steps_other_kernels_equal_the_exchange_loop(golden, pb, case):
 
 @pytest.mark.parametrize("tune", [False, True])
 @pytest.mark.parametrize("epilogue", [0, 2])
-def test_pair_steps_at_odd_y_extents(golden, pb, epilogue, tune):
-    """Even x and odd y extents: the two-row kernel's last row of a patch has no partner, and its +y
-    neighbours lie in the next patch. Odd z extents leave chunks of one and a few planes. Bitwise the
-    exchange + stencil loop (epilogue 0: the plain application)."""
+@pytest.mark.parametrize("widths", [[[16, 24, 64], [15, 17, 3, 8], [16, 33, 3, 17]],
+                                    [[64, 24, 48, 64], [65, 17, 3, 100], [33, 3, 17, 96]]])
+def test_pair_steps_at_odd_y_extents(golden, pb, widths, epilogue, tune):
+    """Even x and odd y extents: the last row of a patch has no partner in the two-row kernel (5.5 M cells;
+    the small level takes one row per thread), and its +y neighbours lie in the next patch. Odd z extents
+    leave chunks of one and a few planes. Bitwise the exchange + stencil loop (epilogue 0: the plain
+    application)."""
     import torch
-    widths = [[16, 24, 64], [15, 17, 3, 8], [16, 33, 3, 17]]
     lv, S, _, u, a, L = _level13(golden, pb, widths, 17)
     b = torch.zeros_like(a)
     h = 1.0 / L[0]
