@@ -117,8 +117,9 @@ __global__ void __launch_bounds__(2 * NXT + 32, relax2_min_blocks(2 * NXT + 32))
     // arithmetic of FP32 levels the three copies (times two groups) outgrow the instruction cache (half of all
     // stalls were instruction fetches), and one copy with about 36 register moves a plane is faster.
     // Measured (B200, Helmholtz pair): 384^3 326 -> 207 us, ending in the update 394 -> 279, from zero 221 ->
-    // 161; 192^3 48.9 -> 38.3.
-    constexpr bool kRoll = sizeof(T) == 4;
+    // 161; 256^3 72.4 -> 69.9; 192^3 48.9 -> 38.3; 128^3 16.5 -> 14.6. Poisson: 384^3 208 -> 153, 128^3 13.9 -> 12.5; at
+    // 192^3 and 256^3 its three copies are no slower (30.9 both; 54.2 against 55.5 rolled) and stay.
+    constexpr bool kRoll = sizeof(T) == 4 && (HELM || N < 192 || N > 256);
     static_assert(NXT % 32 == 0, "groups are whole warps");
     static_assert(!(NORM && MODE != kRelax2Plain), "the norm rides on plain passes only");
     static_assert(!UPD || sizeof(T) == 4, "the update pass belongs to mixed precision");
