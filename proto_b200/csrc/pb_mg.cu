@@ -174,6 +174,21 @@ static AuxSpecs level_aux(const pb_mg* mg, const T* rhs, const T* alpha, const M
     return a;
 }
 
+// Which sweeps of a level below 128 march (k_relax_march); the others take the star kernels. Where the lines
+// lie (B200, us a sweep, star / march): FP64 16^3 2.24 / 2.50, 32^3 2.36 / 2.61, 52^3 3.45 / 3.25, 64^3
+// 4.26 / 3.81, 72^3 5.34 / 5.69, 80^3 6.66 / 6.44 (Helmholtz 7.10 / 7.53), 96^3 8.23 / 6.59, 104^3 9.91 / 10.24,
+// 120^3 12.7 / 13.0; FP32 32^3 2.21 / 2.35, 48^3 2.73 / 2.62, 64^3 4.05 / 3.38, 72^3 5.11 / 4.71, 96^3
+// 6.94 / 5.40, 120^3 10.6 / 9.90. Edges that are no multiple of 8 leave the star kernel's tiles part empty, and
+// edges just above a multiple of 32 the march's lanes.
+template <typename T>
+static bool marches(int n)
+{
+    const bool f32 = sizeof(T) == 4;
+    if (n < 2 || n >= kMarchEdge) return false;
+    if (f32) return n < 48 ? n % 8 != 0 : n <= 64 || n >= 72;
+    return n <= 64 ? n > 56 || (n > 40 && n % 8 != 0) : n > 80 && n <= 96;
+}
+
 template <typename T>
 static int launch_relax(pb_mg* mg, MGLevel<T>& L, bool first, cudaStream_t st)
 {
@@ -182,12 +197,12 @@ static int launch_relax(pb_mg* mg, MGLevel<T>& L, bool first, cudaStream_t st)
         const Walk w = walk_cube(L.n);
         k_relax_first<T><<<walk_grid(w, 1), kWalkThreads, 0, st>>>(L.rhs, L.alpha, L.phi[1 - L.cur], k, w);
         PB_LAUNCH_CHECK();
-    } else if (L.n > 1 && L.n < kMarchEdge) {
-        // lanes along x: the smallest power of two that holds a row, 8 to 32; z chunks for two blocks per SM
-        int lx = 5, zd = 8;
+    } else if (marches<T>(L.n)) {
+        // lanes along x: the smallest power of two that holds a row, 8 to 32
+        int lx = 5;
         while (lx > 3 && (1 << (lx - 1)) >= L.n) lx--;
+        const int zd = L.n < 56 ? 1 : (L.n <= 64 ? 2 : 4);       // planes of a thread
         const int rows = 2 * (256 >> lx), gx = (L.n + (1 << lx) - 1) >> lx, gy = (L.n + rows - 1) / rows;
-        while (zd > 1 && (long long)gx * gy * ((L.n + zd - 1) / zd) < 2LL * cached_sm_count()) zd /= 2;
         const Coefs<T> c = lap7_coefs<T>(is_helm(mg) ? L.hsqinv : mg->p.omega / 6.0);
         const dim3 grid(gx, gy, (L.n + zd - 1) / zd);
         if (is_helm(mg))

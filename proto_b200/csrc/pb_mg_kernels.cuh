@@ -365,10 +365,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_relax_first(const T* __restric
 
 // One sweep of a level too small for the staged kernels (below kMarchEdge), as a march: a thread takes
 // two rows of one x and zd planes, keeps the rows' values at three planes in registers and reads the
-// x neighbours and the two rows beyond from L1-resident rows, so a cell costs four loads and no 64-bit
-// division, and a plane's loads are all in flight together. These sweeps take as long as a launch and
-// two memory latencies; the staged kernel's ring fill and the one-cell kernel's index arithmetic came on
-// top. Same arithmetic as EpiRelax (taps in the Laplacian's order, relax_value).
+// x neighbours and the two rows beyond from L1-resident rows, so a cell costs five loads (six with alpha) and
+// no 64-bit division, and a plane's loads are all in flight together. These sweeps take as long as a launch
+// and two memory latencies. Same arithmetic as EpiRelax (taps in the Laplacian's order, relax_value). Which
+// edges march, and how many planes a thread takes, is measured where it is launched.
 constexpr int kMarchEdge = 128;
 template <typename T, bool HELM>
 __global__ void __launch_bounds__(256) k_relax_march(const T* __restrict__ phi, T* out, const T* __restrict__ rhs,
