@@ -25,8 +25,6 @@
 
 namespace pb {
 
-PB_DEFINE_ERROR_READER(read_error_fas)
-
 constexpr int kFasGhost = 2;      // reach of the operator
 
 // index of cell (x, y, z) of a plain n^3 field, and of a level's state (x and y may be ghosts)
@@ -725,7 +723,6 @@ int pb_fas_solve(pb_fas* m, const double* force, double* phi, int max_iter, doub
     k_fas_unpack<<<walk_grid(wv, 1), kWalkThreads, 0, st>>>(T.u[T.cur], phi, T.n, wv);
     PB_LAUNCH_CHECK();
     PB_CUDA(cudaStreamSynchronize(st));
-    if (read_error_fas() > 0) return PB_ERR_DEVICE;
     if (iters) *iters = it;
     return PB_OK;
 }

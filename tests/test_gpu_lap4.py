@@ -50,3 +50,21 @@ def test_fas_level_shapes(pb, port, n, levels, cycles):
     n2, h2 = port.mg_fas(n, levels, cycles, 1e-14, force, want)
     assert it == n2 and hist == list(h2)
     assert np.array_equal(phi.cpu().numpy(), want)
+
+
+def test_fas_solve_waits_for_its_own_stream_only(pb):
+    """A solve on a stream of its own ends while the default stream is still busy."""
+    import torch
+    m, side = pb.FAS(32, 3), torch.cuda.Stream()
+    f = torch.from_numpy(np.random.default_rng(2).uniform(-1, 1, 32 ** 3)).cuda()
+    phi = torch.zeros_like(f)
+    torch.cuda.synchronize()
+    want = m.solve(f, phi, max_iter=3, tol=0.0, stream=side.cuda_stream)     # captures its graphs
+    phi.zero_()
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(1 << 30)                                               # about half a second
+    busy.record()
+    assert m.solve(f, phi, max_iter=3, tol=0.0, stream=side.cuda_stream) == want
+    assert not busy.query()
+    torch.cuda.synchronize()
