@@ -94,7 +94,10 @@ def _call(name, *args):
     if _CALLS is None:
         L = lib()
         _CALLS = {k: ctypes.CFUNCTYPE(_c_int, *v)((k, L)) for k, v in _PROTOTYPES.items()}
-    status = _CALLS[name](*args)
+    try:
+        status = _CALLS[name](*args)
+    except ctypes.ArgumentError as e:      # an argument that its C type does not take
+        raise TypeError(str(e)) from None
     if status != 0:
         raise ProtoError(status, "pb_stencil_apply" if name in ("pb_stencil_apply_f64", "pb_stencil_apply_f32") else name)
 
@@ -145,6 +148,8 @@ def _check(status, where):
 def _raw_stream(stream):
     """The stream argument of _call: the caller's, or torch's current one."""
     if stream is not None:
+        if type(stream) is not int:
+            _vp(stream)      # refuses what is no handle (a pointer argument would take bytes and text)
         return stream
     import torch
     return torch.cuda.current_stream().cuda_stream

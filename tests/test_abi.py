@@ -147,3 +147,30 @@ def test_wait_expiry_hook_validates_arguments():
     assert L.pb_debug_wait_expiry(ctypes.c_uint(0), ctypes.byref(e), None) == -1
     assert L.pb_debug_wait_expiry(ctypes.c_uint(1000), None, None) == -1
     assert L.pb_debug_wait_expiry(ctypes.c_uint((1 << 24) + 1), ctypes.byref(e), None) == -1
+
+
+@pytest.mark.parametrize("stream", ["0", b"stream", 0.0, ctypes.c_void_p(3), (ctypes.c_int * 2)()])
+def test_per_call_entry_points_refuse_what_is_no_stream(stream):
+    """Refused before the library is called: text, bytes and arrays are no stream handles, although a pointer
+    argument would take them."""
+    class Null:
+        def data_ptr(self):
+            return 0
+    with pytest.raises(TypeError):
+        pb.boxdata_scalar(pb.OP_ADD, Null(), pb.Box.cube(4), 1.0, stream=stream)
+
+
+def test_per_call_entry_points_raise_type_errors():
+    """An argument of the wrong type is a TypeError, as from the ctypes constructors, and nothing is called."""
+    class Null:
+        def data_ptr(self):
+            return 0
+    b = pb.Box.cube(4)
+    with pytest.raises(TypeError):
+        pb.boxdata_scalar("add", Null(), b, 1.0, stream=0)
+    with pytest.raises(TypeError):
+        pb.boxdata_scalar(pb.OP_ADD, Null(), b, "1.0", stream=0)
+    with pytest.raises(TypeError):
+        pb.reduce(1.5, Null(), b, stream=0)
+    with pytest.raises(pb.ProtoError):         # right types, null field: the library's own refusal
+        pb.boxdata_scalar(pb.OP_ADD, Null(), b, 1.0, stream=0)
