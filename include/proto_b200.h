@@ -84,7 +84,8 @@ int pb_stencil_apply_f32(const pb_stencil* s, const float* src, pb_box src_box,
  * points each consumer thread computes: (ty, yb, xv) one of (8,1,1), (8,2,1), (8,2,2), (4,2,2),
  * or (8,2,0), the default, which uses xv = 1 for Stencil::apply and xv = 2 for the multigrid
  * sweeps (xv = 2 applies to boxes of even x extent; others use xv = 1). min_tma_points < 0 keeps
- * the current threshold. */
+ * the current threshold. Two-sweep passes, and the sweeps of levels below 128 that march (the
+ * edges where that was measured faster), are kernels of their own that no knob shapes. */
 int pb_star_tune_set(int mode, int zc, int ty, int yb, int xv, long long min_tma_points);
 /* Depth of the TMA kernel's shared-memory ring (0: up to 2R+4 planes, 2R+3 with two x points per
  * thread, as deep as two CTAs per SM allow; else 2R+1..16) and whether
@@ -123,7 +124,8 @@ int pb_forall_axpby_f64(double* out, pb_box out_box, const double* x, pb_box x_b
  * op: 0 Max (initial value DBL_MIN, as the reference), 1 Min, 2 Abs (absMax), 3 Sum, 4 SumAbs,
  * 5 SumSquare, over 'region' of a field on 'box' (empty region = whole box), one component.
  * pb_reduce_f64 waits for the result (Reduction::fetch); the _async form leaves the result in
- * device memory. Max/Min/Abs are exact; sums use a fixed two-level tree (deterministic run to run).
+ * device memory. Max/Min/Abs are exact; sums use a fixed two-level tree (deterministic run to run; its
+ * order follows the region's extents and may change between versions, in a sum's last places).
  * Both may be called from several threads and on several streams at once: each call in flight has
  * scratch of its own (3 KB, kept for later calls). A captured pb_reduce_async_f64 takes scratch that
  * lives as long as the graph. */

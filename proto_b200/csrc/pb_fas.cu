@@ -189,7 +189,7 @@ struct EpiFasRestrict {
 };
 
 // fine correction: u += -(c0 - uc) of the cell's coarse cell (c0: the coarse state as it was averaged,
-// uc: as the coarse cycle left it). A row walk with four planes' loads in flight.
+// uc: as the coarse cycle left it). An item walk with four planes' loads in flight.
 template <bool SMALL>
 __global__ void __launch_bounds__(kWalkThreads) k_fas_correct(double* u, const double* __restrict__ c0,
                                                               const double* __restrict__ uc, int nf, Walk w)

@@ -12,8 +12,9 @@
 //     coefficients are +cp and -cp); the z faces are carried from plane to plane, the y face between
 //     the two rows is computed once;
 //   * the leading "0 +" of a flux only decides the sign of a zero, which the final 0 + t removes.
-// That leaves 41 operations and 7 loads a cell (the z window keeps values, and their products are formed
-// again as they are needed: three operations a cell for 28 registers). With two resident blocks per SM
+// That leaves 38 operations and 7 loads a cell (22 operations that the two rows share and 27 for each; the z
+// window keeps values, and their products are formed again as they are needed: three operations a cell for
+// 28 registers). With two resident blocks per SM
 // only four warps share a scheduler, so no load may be waited for: a plane's neighbours, and what the
 // epilogue needs, are loaded one plane ahead. All loads are 8 bytes wide from L1-resident rows, so odd
 // sizes and any alignment run the same code. Two cells beyond the range are
