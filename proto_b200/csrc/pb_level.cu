@@ -493,7 +493,12 @@ __global__ void __launch_bounds__(kLevelThreads / ROWS, ROWS == 2 ? 5 : 4) k_lev
             // rows y-2 .. y+ROWS+1 of this pair
             double2 yy[4 + ROWS];
 #pragma unroll
-            for (int r = 0; r < 4 + ROWS; r++) yy[r] = r < 2 || r >= 2 + ROWS ? ring2(pl + (r - 2) * BX) : w[r < 2 ? 0 : r - 2 < ROWS ? r - 2 : 0][wc];
+            for (int r = 0; r < 2; r++) {
+                yy[r] = ring2(pl + (r - 2) * BX);
+                yy[2 + ROWS + r] = ring2(pl + (ROWS + r) * BX);
+            }
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) yy[2 + r] = w[r][wc];
 #pragma unroll
             for (int r = 0; r < ROWS; r++) {
                 const double2 xm = ring2(pl + r * BX - 2);   // x-2, x-1
